@@ -38,14 +38,17 @@ CCTAGB_HD inline int link_shift(float angle)
 }
 
 // Vote.cpp:329-344: convexity test between the oldest and the newest angle of
-// the window (full: the window holds windowSize angles).
+// the window (full: the window holds windowSize angles).  With t = dir * (back
+// - front) the reference asks for sin t < 0 (full), else for (sin t < -0.707f
+// and cos t > 0) or (sin t < 0 and cos t < 0).  The angles lie in [0, 2 pi),
+// so |t| < 2 pi, where those are the intervals below: their ends are the first
+// and last floats at which pm::sinf_ and pm::cosf_ meet the conditions
+// (tests/cpp/convexity_test.cpp walks the floats around them).
 CCTAGB_HD inline bool link_convexity_lost(float front, float back, bool full, int dir)
 {
-    const float d = back - front;
-    if (full) return float(dir) * pm::sinf_(d) < 0.0f;
-    const float s = float(dir) * pm::sinf_(d);
-    const float c = pm::cosf_(d);
-    return (s < -0.707f && c > 0.f) || (s < 0.f && c < 0.f);
+    const float t = float(dir) * (back - front);
+    if (full) return (t < 0.0f && t >= -3.1415925f) || t >= 3.14159274f;
+    return (t <= -0.785247266f && t >= -3.1415925f) || (t >= 3.14159274f && t <= 5.49793768f);
 }
 
 // Vote.cpp:352: running mean of the votes received along the segment.
