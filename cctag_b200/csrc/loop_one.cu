@@ -20,7 +20,11 @@
 //                 128 random draws evaluated at once and accepted in draw
 //                 order; the draws' random stream is generated in parallel
 //                 with the PCG jump-ahead;
-// k_pack          the kept candidates' filtered children, packed for download.
+// k_pack          the kept candidates' filtered children, packed for download;
+// k_refit_hull, k_refit, k_refit_pack
+//                 one block per coarse-level marker: its level-0 hull points
+//                 (Multiresolution.cpp:319-401), the same outlier removal on
+//                 them, packed for download.
 #include "loop_one.hpp"
 
 #include <algorithm>
@@ -542,143 +546,249 @@ __device__ __forceinline__ int draw_from(const uint8_t* mods, int p0, int g[5])
     return q;
 }
 
-// Whether the (weighted) distance d(Q, p) * w of dist_point_ellipse is below
-// S, decided exactly: an estimate with the fast reciprocal settles the cases
-// that are more than 2^-16 (relative) away from S; the rest are computed with
+// How many of the np (weighted) distances d(Q, p) * w of dist_point_ellipse are
+// below S, exactly: an estimate with the approximate reciprocal (relative error
+// below 2^-20) settles the points that are more than 2e-5 (relative) away from
+// S; if any point is closer, or its estimate is not finite or its denominator
+// beyond the reciprocal's range (or S near the denormals), all are counted with
 // the IEEE expression.
-__device__ __forceinline__ bool dist_below(const geo::Mat3& Q, float x, float y, bool weighted, float w, float S)
+__device__ __forceinline__ int count_below(const geo::Mat3& Q, const geo::Pt* pts, const float* wts, int np,
+                                           bool weighted, float S)
 {
-    const float aux0 = x * x, aux1 = 2 * x * y, aux2 = 2 * x, aux3 = y * y, aux4 = 2 * y;
-    const float t1 = x * Q.m[0][0] + y * Q.m[0][1] + Q.m[0][2];
-    const float t2 = x * Q.m[0][1] + y * Q.m[1][1] + Q.m[1][2];
-    const float denom = t1 * t1 + t2 * t2;
-    const float dot = aux0 * Q.m[0][0] + aux1 * Q.m[0][1] + aux2 * Q.m[0][2] + aux3 * Q.m[1][1] + aux4 * Q.m[1][2] +
-                      Q.m[2][2];
-    const float dd = dot * dot;
-    float v = dd * __frcp_rn(denom);
-    if (weighted) v *= w;
-    if (v < S * 0.99998f) return true;
-    if (v > S * 1.00002f && v <= 3.4e38f) return false;  // an infinite estimate is settled exactly
-    float d = dd / denom;
-    if (weighted) d *= w;
-    return d < S;
+    const float lo = S * 0.99998f, hi = S * 1.00002f;
+    int below = 0;
+    bool close = !(S > 1e-30f);
+#pragma unroll 4
+    for (int i = 0; i < np; ++i) {
+        const float x = pts[i].x, y = pts[i].y;
+        const float aux0 = x * x, aux1 = 2 * x * y, aux2 = 2 * x, aux3 = y * y, aux4 = 2 * y;
+        const float t1 = x * Q.m[0][0] + y * Q.m[0][1] + Q.m[0][2];
+        const float t2 = x * Q.m[0][1] + y * Q.m[1][1] + Q.m[1][2];
+        const float denom = t1 * t1 + t2 * t2;
+        const float dot = aux0 * Q.m[0][0] + aux1 * Q.m[0][1] + aux2 * Q.m[0][2] + aux3 * Q.m[1][1] +
+                          aux4 * Q.m[1][2] + Q.m[2][2];
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(denom));
+        float v = dot * dot * r;
+        if (weighted) v *= wts[i];
+        const bool less = v < lo, more = v > hi && v <= 3.4e38f;
+        close = close || !(less || more) || !(denom < 1e37f);
+        below += less ? 1 : 0;
+    }
+    if (close) {
+        below = 0;
+        for (int i = 0; i < np; ++i) {
+            float d = geo::dist_point_ellipse(Q, pts[i].x, pts[i].y);
+            if (weighted) d *= wts[i];
+            below += d < S ? 1 : 0;
+        }
+    }
+    return below;
+}
+
+constexpr int kRawPer = kRawPool / kFilterThreads;  // random outputs per thread
+constexpr int kRawEnd = kRawPool;                    // start position past the last output
+constexpr int kRawDead = kRawPool + 1;               // ... and after a draw the pool does not hold whole
+constexpr int kFirstMedians = 12;                    // draws of the first batch whose median is taken outright
+
+// Shared state of one outlier removal.
+struct LmedsShared {
+    geo::Pt pts[kLmedsMaxPts];
+    float wts[kLmedsMaxPts];
+    uint32_t raws[kRawPool];
+    alignas(8) uint8_t mods[kRawPool + 16];          // raws mod np; 255 past the end
+    int16_t next[kRawDead + 1];                      // where the draw at a position ends
+    int16_t jump[2][kRawDead + 1];                   // ... 2^b draws on
+    int8_t perms[kFilterThreads][5];
+    int kinds[kFilterThreads];
+    float svals[kFilterThreads];
+    float Q[kFilterThreads][9];
+    float bestQ[9];
+    long long target[kLmedsMaxPts + 1];
+    int npts, done, nd, counter, draws, warpCnt[4][kFilterThreads / 32];
+    float sm;
+    unsigned long long state, inc;
+};
+
+// The draws (Statistic.cpp:16-29 rand_5_k) held by the pool of random outputs
+// in S.mods: a draw consumes outputs until it has 5 distinct residues.  Every
+// position's draw length is found in parallel (the residues of the next
+// outputs as bits of a 64-bit word, np <= 64); the k-th draw's start is the
+// k-fold chain of those lengths from position 0, followed by pointer doubling,
+// one thread per draw.  Sets S.nd, S.perms and the stream's next state.
+// (A chain walked by one thread, with the lengths read byte by byte, took
+// 30 k of a batch's 75 k cycles.)
+__device__ __forceinline__ void lmeds_draws(LmedsShared& S)
+{
+    const int tid = threadIdx.x;
+    uint64_t bit[kRawPer + 11];
+#pragma unroll
+    for (int k = 0; k < kRawPer + 11; ++k) {
+        const int v = S.mods[min(tid * kRawPer + k, kRawPool + 15)];
+        bit[k] = v < 64 ? 1ull << v : 0ull;
+    }
+#pragma unroll
+    for (int k = 0; k < kRawPer; ++k) {
+        const int p = tid * kRawPer + k;
+        uint64_t m = bit[k] | bit[k + 1] | bit[k + 2] | bit[k + 3] | bit[k + 4];
+        int len = 5, have = __popcll(m);
+#pragma unroll
+        for (int q = 5; q < 12; ++q) {
+            len += have < 5 ? 1 : 0;
+            m |= bit[k + q];
+            have = have < 5 ? __popcll(m) : have;
+        }
+        int end = p + len;
+        if (have < 5 || end > kRawEnd) {  // longer than 12 outputs, or past the pool
+            int g[5];
+            const int q = draw_from(S.mods, p, g);
+            end = q > 0 ? q : kRawDead;
+        }
+        S.next[p] = S.jump[0][p] = int16_t(end);
+    }
+    if (tid < 2) S.next[kRawEnd + tid] = S.jump[0][kRawEnd + tid] = S.jump[1][kRawEnd + tid] = int16_t(kRawDead);
+    __syncthreads();
+    int p = 0;  // start of draw tid
+    for (int b = 0; 1 << b < kFilterThreads; ++b) {
+        const int16_t* J = S.jump[b & 1];
+        if (tid >> b & 1) p = J[p];
+        int16_t* N = S.jump[(b & 1) ^ 1];
+#pragma unroll
+        for (int k = 0; k < kRawPer; ++k) {
+            const int q = k * kFilterThreads + tid;
+            N[q] = J[J[q]];
+        }
+        __syncthreads();
+    }
+    const bool whole = p < kRawEnd && S.next[p] <= kRawEnd;  // and so are all draws before it
+    const int nd = __syncthreads_count(whole);
+    if (whole) {
+        int g[5];
+        const int end = draw_from(S.mods, p, g);
+#pragma unroll
+        for (int i = 0; i < 5; ++i) S.perms[tid][i] = int8_t(g[i]);
+        if (tid == nd - 1) {
+            geo::Pcg32 r;
+            r.state = S.state;
+            r.inc = S.inc;
+            r.advance(uint64_t(end));
+            S.state = r.state;
+        }
+    }
+    if (tid == 0) S.nd = nd;
+}
+
+// The median (rank np / 2, NaN last) of draw d's distances, by a warp: two
+// points per lane, then a 64-key bitonic sort.
+__device__ __forceinline__ float lmeds_median(const LmedsShared& S, int d, int np, bool weighted, int lane)
+{
+    geo::Mat3 Q;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Q.m[k / 3][k % 3] = S.Q[d][k];
+    uint32_t key[2] = {0xffffffffu, 0xffffffffu};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;
+        if (i < np) {
+            float v = geo::dist_point_ellipse(Q, S.pts[i].x, S.pts[i].y);
+            if (weighted) v *= S.wts[i];
+            key[h] = geo::order_key(v);
+        }
+    }
+    bitonic64(key[0], key[1], lane);
+    const int r = np / 2;
+    return key_value(__shfl_sync(kFull, r < 32 ? key[0] : key[1], r & 31));
 }
 
 // Block-wide outlierRemoval (Vote.cpp:414-576) with maxSize 60 over the n
 // edge points idx[0, n) of level L: LMedS ellipse from random 5-point subsets
-// of a regular subsample, drawn from `rng`, kDrawsPerBatch at a time and
+// of a regular subsample, drawn from `rng`, kFilterThreads at a time and
 // accepted in draw order; then idx is compacted in place (order kept) to the
 // points whose distance (times 255 / |gradient| when weighted) is below
 // threshold * the best median.  Returns their number (0 when fewer than 5
 // points are subsampled).  Every thread of the block must call it.
+//
+// Latency-bound (one block of 4 warps per candidate, 1-3 batches of draws).  A
+// draw's median costs a warp some 900 cycles, so only draws that can improve
+// get one: those with enough distances below a median known to come before
+// them, the first batch's bound being the least of its first kFirstMedians.
+// Measured (1080p frame, cold): k_filter 124 us with the draws chained by one
+// thread, a median per usable draw and the children gathered by one warp, 58 us
+// now (3840x2160 clutter: 149 us and 63 us); the re-fit's removal 46 us.
 __device__ int lmeds_outliers(const LoopOneLevel& L, int32_t* idx, int n, bool weighted, float threshold,
                               const geo::Pcg32 rng0, int32_t* err)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __shared__ geo::Pt pts[kLmedsMaxPts];
-    __shared__ float wts[kLmedsMaxPts];
-    __shared__ uint32_t raws[kRawPool];
-    __shared__ uint8_t mods[kRawPool];
-    __shared__ int16_t lens[kRawPool];
-    __shared__ uint32_t keysAll[kLmedsMaxPts * kFilterThreads];
-    __shared__ int16_t starts[kFilterThreads];
-    __shared__ int8_t perms[kFilterThreads][5];
-    __shared__ int kinds[kFilterThreads];
-    __shared__ float svals[kFilterThreads];
-    __shared__ float sQ[kFilterThreads][9];
-    __shared__ float bestQ[9];
-    __shared__ int sNpts, sDone, sNd, sCounter, sDraws, sWarpCnt[kFilterThreads / 32];
-    __shared__ float sSm;
-    __shared__ unsigned long long sState, sInc;
+    __shared__ LmedsShared S;
     const int nchild = n;
     int32_t* children = idx;
     // The reference scans the children and takes child i when i equals
     // size_t(float(k) * step) for the next k: the taken indices are those
     // targets while they increase strictly and stay below nchild.
     const int nSub = min(nchild, 60);
-    __shared__ long long sTarget[kLmedsMaxPts + 1];
-    if (nSub >= 5 && tid <= kLmedsMaxPts) {
+    if (nSub < 5) return 0;
+    if (tid <= kLmedsMaxPts) {
         const float step = float(nchild) / float(nSub);
-        sTarget[tid] = (long long)size_t(float(size_t(tid)) * step);
+        S.target[tid] = (long long)size_t(float(size_t(tid)) * step);
     }
+    if (tid < 16) S.mods[kRawPool + tid] = 255;
     __syncthreads();
+    {
+        // the targets taken: a prefix of them
+        const bool take = tid <= kLmedsMaxPts && S.target[tid] < nchild && (tid == 0 || S.target[tid] > S.target[tid - 1]);
+        const unsigned m = __ballot_sync(kFull, take);
+        if (lane == 0) S.warpCnt[0][warp] = m == kFull ? 32 : __ffs(~m) - 1;
+    }
     if (tid == 0) {
-        int np = 0;
-        if (nSub >= 5) {
-            while (np <= kLmedsMaxPts && sTarget[np] < nchild && (np == 0 || sTarget[np] > sTarget[np - 1])) ++np;
-            if (np > kLmedsMaxPts) atomicOr(err, kLoopOneErrPoints);
-        }
-        sNpts = np;
-        for (int k = 0; k < 9; ++k) bestQ[k] = 0.f;
-        sSm = 10000000.0f;
-        sDone = 0;
-        sCounter = 0;
-        sDraws = 0;
-        sState = rng0.state;
-        sInc = rng0.inc;
+        for (int k = 0; k < 9; ++k) S.bestQ[k] = 0.f;
+        S.sm = 10000000.0f;
+        S.done = 0;
+        S.counter = 0;
+        S.draws = 0;
+        S.state = rng0.state;
+        S.inc = rng0.inc;
     }
     __syncthreads();
-    const int np = sNpts;
-    if (np <= kLmedsMaxPts && tid < np) {
-        const int e = children[sTarget[tid]];
-        pts[tid] = {float(px_(L, e)), float(py_(L, e))};
-        wts[tid] = 255.f / gnorm(L, e);
+    int np = 0;
+    for (int w = 0; w < kFilterThreads / 32; ++w) {
+        np += S.warpCnt[0][w];
+        if (S.warpCnt[0][w] < 32) break;
+    }
+    if (np > kLmedsMaxPts) {
+        if (tid == 0) atomicOr(err, kLoopOneErrPoints);
+        return 0;
+    }
+    if (tid < np) {
+        const int e = children[S.target[tid]];
+        S.pts[tid] = {float(px_(L, e)), float(py_(L, e))};
+        S.wts[tid] = 255.f / gnorm(L, e);
     }
     __syncthreads();
-    if (nSub < 5 || np > kLmedsMaxPts) return 0;
     // ... then random 5-point conics, 128 draws at a time, accepted in order.
     const uint32_t rejectBelow = uint32_t(-uint32_t(np)) % uint32_t(np);
-    while (!sDone) {
-        // the next kRawPool outputs of the candidate's stream, 8 per thread
+    for (bool first = true; !S.done; first = false) {
+        // the next kRawPool outputs of the candidate's stream, 8 per thread.
+        // A bounded draw rejects an output only below 2^32 mod np (< 64 of
+        // 2^32 values).
+        bool rejects = false;
         {
             geo::Pcg32 g;
-            g.state = sState;
-            g.inc = sInc;
-            g.advance(uint64_t(tid) * (kRawPool / kFilterThreads));
-            for (int k = 0; k < kRawPool / kFilterThreads; ++k) {
+            g.state = S.state;
+            g.inc = S.inc;
+            g.advance(uint64_t(tid) * kRawPer);
+            uint32_t packed[2] = {0u, 0u};
+#pragma unroll
+            for (int k = 0; k < kRawPer; ++k) {
                 const uint32_t r = g.next();
-                raws[tid * (kRawPool / kFilterThreads) + k] = r;
-                mods[tid * (kRawPool / kFilterThreads) + k] = uint8_t(r % uint32_t(np));
+                S.raws[tid * kRawPer + k] = r;
+                packed[k >> 2] |= (r % uint32_t(np)) << (8 * (k & 3));
+                rejects = rejects || r < rejectBelow;
             }
+            *reinterpret_cast<uint2*>(S.mods + tid * kRawPer) = make_uint2(packed[0], packed[1]);
         }
-        // Statistic.cpp:16-29 rand_5_k on that stream, as many whole draws as
-        // it holds.  A bounded draw rejects an output only below 2^32 mod np
-        // (< 64 of 2^32 values): when the pool holds none, a draw consumes
-        // outputs until it has 5 distinct residues, so each position's draw
-        // length is found in parallel and the draws chained from position 0.
-        bool rejects = false;
-        for (int k = 0; k < kRawPool / kFilterThreads; ++k)
-            rejects = rejects || raws[tid * (kRawPool / kFilterThreads) + k] < rejectBelow;
         rejects = __syncthreads_or(rejects);
         if (!rejects) {
-            for (int k = 0; k < kRawPool / kFilterThreads; ++k) {
-                const int p0 = tid * (kRawPool / kFilterThreads) + k;
-                int g[5];
-                const int q = draw_from(mods, p0, g);
-                lens[p0] = int16_t(q > 0 ? q - p0 : -1);
-            }
-            __syncthreads();
-            if (tid == 0) {
-                int ptr = 0, nd = 0;
-                while (nd < kFilterThreads && ptr < kRawPool && lens[ptr] > 0) {
-                    starts[nd++] = int16_t(ptr);
-                    ptr += lens[ptr];
-                }
-                if (nd == 0) atomicOr(err, kLoopOneErrRandom);
-                sNd = nd;
-                geo::Pcg32 g;
-                g.state = sState;
-                g.inc = sInc;
-                g.advance(uint64_t(ptr));
-                sState = g.state;
-            }
-            __syncthreads();
-            if (tid < sNd) {
-                int g[5];
-                draw_from(mods, starts[tid], g);
-#pragma unroll
-                for (int i = 0; i < 5; ++i) perms[tid][i] = int8_t(g[i]);
-            }
+            lmeds_draws(S);
         } else if (tid == 0) {
             int ptr = 0, nd = 0;
             while (nd < kFilterThreads) {
@@ -691,8 +801,8 @@ __device__ int lmeds_outliers(const LoopOneLevel& L, int32_t* idx, int n, bool w
                             complete = false;
                             break;
                         }
-                        const uint32_t raw = raws[ptr];
-                        const int r = mods[ptr];
+                        const uint32_t raw = S.raws[ptr];
+                        const int r = S.mods[ptr];
                         ++ptr;
                         if (raw < rejectBelow) continue;
                         bool seen = false;
@@ -706,67 +816,57 @@ __device__ int lmeds_outliers(const LoopOneLevel& L, int32_t* idx, int n, bool w
                     ptr = start;
                     break;
                 }
-                for (int i = 0; i < 5; ++i) perms[nd][i] = int8_t(perm[i]);
+                for (int i = 0; i < 5; ++i) S.perms[nd][i] = int8_t(perm[i]);
                 ++nd;
             }
-            if (nd == 0) atomicOr(err, kLoopOneErrRandom);
-            sNd = nd;
+            S.nd = nd;
             geo::Pcg32 g;
-            g.state = sState;
-            g.inc = sInc;
+            g.state = S.state;
+            g.inc = S.inc;
             g.advance(uint64_t(ptr));
-            sState = g.state;
+            S.state = g.state;
         }
         __syncthreads();
-        const int nd = sNd;
-        if (nd == 0) break;
-        const float SmStart = sSm;
-        {
-            const bool valid = tid < nd;
-            geo::Mat3 Q = geo::Mat3::zero();
-            int kind = kDrawNotReal;
-            bool needS = false;
-            if (valid) {
-                int perm[5];
-                for (int i = 0; i < 5; ++i) perm[i] = perms[tid][i];
-                kind = cand::lmeds_conic(pts, perm, Q);
-                if (kind == kDrawUsable) {
-                    int below = 0;
-#pragma unroll 4
-                    for (int i = 0; i < np; ++i) below += dist_below(Q, pts[i].x, pts[i].y, weighted, wts[i], SmStart);
-                    // no median below the best so far: it cannot improve (Sm only decreases)
-                    if (below >= np / 2 + 1) {
-                        needS = true;
-                        uint32_t* keys = keysAll + tid;  // column tid of a [kLmedsMaxPts][kFilterThreads] array
-                        for (int i = 0; i < np; ++i) {
-                            float d = geo::dist_point_ellipse(Q, pts[i].x, pts[i].y);
-                            if (weighted) d *= wts[i];
-                            keys[i * kFilterThreads] = geo::order_key(d);
-                        }
-                    } else {
-                        kind = kDrawNoGain;
-                    }
+        const int nd = S.nd;
+        if (nd == 0) {
+            if (tid == 0) atomicOr(err, kLoopOneErrRandom);
+            break;
+        }
+        geo::Mat3 Q = geo::Mat3::zero();
+        int kind = kDrawNotReal;
+        if (tid < nd) {
+            int perm[5];
+            for (int i = 0; i < 5; ++i) perm[i] = S.perms[tid][i];
+            kind = cand::lmeds_conic(S.pts, perm, Q);
+            S.kinds[tid] = kind;
+            S.svals[tid] = 0.f;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) S.Q[tid][k] = Q.m[k / 3][k % 3];
+        }
+        __syncthreads();
+        float bound = S.sm;
+        if (first) {
+            for (int d = warp; d < min(nd, kFirstMedians); d += kFilterThreads / 32)
+                if (S.kinds[d] == kDrawUsable) {
+                    const float med = lmeds_median(S, d, np, weighted, lane);
+                    if (lane == 0) S.svals[d] = med;
                 }
-            }
-            // medians (rank np / 2, NaN last) of the draws that need one, a draw at
-            // a time by the whole warp: a 64-key bitonic sort of its column
-            __syncwarp();
-            float S = 0.f;
-            for (unsigned m = __ballot_sync(kFull, needS); m; m &= m - 1) {
-                const int src = __ffs(m) - 1;
-                const uint32_t* col = keysAll + (warp * 32 + src);
-                uint32_t ka = lane < np ? col[lane * kFilterThreads] : 0xffffffffu;
-                uint32_t kb = lane + 32 < np ? col[(lane + 32) * kFilterThreads] : 0xffffffffu;
-                bitonic64(ka, kb, lane);
-                const int r = np / 2;
-                const uint32_t v = __shfl_sync(kFull, r < 32 ? ka : kb, r & 31);
-                if (lane == src) S = key_value(v);
-            }
-            if (valid) {
-                kinds[tid] = kind;
-                svals[tid] = S;
-                for (int k = 0; k < 9; ++k) sQ[tid][k] = Q.m[k / 3][k % 3];
-            }
+            __syncthreads();
+            for (int d = 0; d < min(nd, kFirstMedians); ++d)
+                if (S.kinds[d] == kDrawUsable) bound = fminf(bound, S.svals[d]);
+        }
+        // the draws that may improve: more than half of their distances are
+        // below a median that comes before them
+        bool needS = false;
+        if (kind == kDrawUsable && tid < nd && !(first && tid < kFirstMedians)) {
+            needS = count_below(Q, S.pts, S.wts, np, weighted, bound) >= np / 2 + 1;
+            if (!needS) S.kinds[tid] = kDrawNoGain;
+        }
+        __syncwarp();
+        for (unsigned m = __ballot_sync(kFull, needS); m; m &= m - 1) {
+            const int d = warp * 32 + __ffs(m) - 1;
+            const float med = lmeds_median(S, d, np, weighted, lane);
+            if (lane == 0) S.svals[d] = med;
         }
         __syncthreads();
         // Acceptance in draw order (Vote.cpp:478-545) by warp 0, 32 draws at a
@@ -776,15 +876,15 @@ __device__ int lmeds_outliers(const LoopOneLevel& L, int32_t* idx, int n, bool w
         // loop stops before the first draw at which it has reached 70 (or the
         // draws 7000).
         if (warp == 0) {
-            int counter = sCounter, draws = sDraws, best = -1;
-            float Sm = sSm;
+            int counter = S.counter, draws = S.draws, best = -1;
+            float Sm = S.sm;
             bool stopped = false;
             for (int c0 = 0; c0 < nd && !stopped; c0 += 32) {
                 const int j = c0 + lane;
                 const bool valid = j < nd;
-                const int kind = valid ? kinds[j] : kDrawNotReal;
+                const int kind = valid ? S.kinds[j] : kDrawNotReal;
                 const bool usable = valid && kind == kDrawUsable;
-                const float Sj = usable ? svals[j] : __int_as_float(0x7f800000);
+                const float Sj = usable ? S.svals[j] : __int_as_float(0x7f800000);
                 float incl = Sj;
                 for (int o = 1; o < 32; o <<= 1) {
                     const float v = __shfl_up_sync(kFull, incl, o);
@@ -822,40 +922,56 @@ __device__ int lmeds_outliers(const LoopOneLevel& L, int32_t* idx, int n, bool w
                 draws += js;
                 stopped = stopM != 0;
             }
+            if (best >= 0 && lane < 9) S.bestQ[lane] = S.Q[best][lane];
             if (lane == 0) {
-                if (best >= 0)
-                    for (int k = 0; k < 9; ++k) bestQ[k] = sQ[best][k];
-                sCounter = counter;
-                sDraws = draws;
-                sSm = Sm;
-                if (stopped || !(counter < 70 && draws < 7000)) sDone = 1;
+                S.counter = counter;
+                S.draws = draws;
+                S.sm = Sm;
+                if (stopped || !(counter < 70 && draws < 7000)) S.done = 1;
             }
         }
         __syncthreads();
     }
-    // the children whose weighted distance is below threshold * median, in order
+    // the children whose weighted distance is below threshold * median, in
+    // order, four per thread at once so that their loads overlap
     geo::Mat3 Q;
-    for (int k = 0; k < 9; ++k) Q.m[k / 3][k % 3] = bestQ[k];
-    const float thr = threshold * sSm;
+    for (int k = 0; k < 9; ++k) Q.m[k / 3][k % 3] = S.bestQ[k];
+    const float thr = threshold * S.sm;
     int nflt = 0;
-    for (int c0 = 0; c0 < nchild; c0 += kFilterThreads) {
-        const int i = c0 + tid;
-        int e = -1;
-        if (i < nchild) e = children[i];
-        __syncthreads();  // every element of the chunk read before any is overwritten
-        bool pass = false;
-        if (e >= 0) {
-            float d = geo::dist_point_ellipse(Q, float(px_(L, e)), float(py_(L, e)));
-            if (weighted) d = d * 255 / gnorm(L, e);
-            pass = d < thr;
+    for (int c0 = 0; c0 < nchild; c0 += 4 * kFilterThreads) {
+        int e[4];
+        bool pass[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const int i = c0 + h * kFilterThreads + tid;
+            e[h] = i < nchild ? children[i] : -1;
         }
-        const unsigned mask = __ballot_sync(kFull, pass);
-        if (lane == 0) sWarpCnt[warp] = __popc(mask);
-        __syncthreads();
-        int off = nflt;
-        for (int w = 0; w < warp; ++w) off += sWarpCnt[w];
-        if (pass) children[off + __popc(mask & ((1u << lane) - 1u))] = e;
-        for (int w = 0; w < kFilterThreads / 32; ++w) nflt += sWarpCnt[w];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            pass[h] = false;
+            if (e[h] >= 0) {
+                float d = geo::dist_point_ellipse(Q, float(px_(L, e[h])), float(py_(L, e[h])));
+                if (weighted) d = d * 255 / gnorm(L, e[h]);
+                pass[h] = d < thr;
+            }
+        }
+        unsigned mask[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            mask[h] = __ballot_sync(kFull, pass[h]);
+            if (lane == 0) S.warpCnt[h][warp] = __popc(mask[h]);
+        }
+        __syncthreads();  // and every element of the chunk read before any is overwritten
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            int off = nflt;
+            for (int w = 0; w < kFilterThreads / 32; ++w) {
+                const int c = S.warpCnt[h][w];
+                off += w < warp ? c : 0;
+                nflt += c;
+            }
+            if (pass[h]) children[off + __popc(mask[h] & ((1u << lane) - 1u))] = e[h];
+        }
         __syncthreads();
     }
     return nflt;
@@ -866,7 +982,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter(LoopOneArgs a)
 {
     const int l = blockIdx.x / a.n2max, rank = blockIdx.x % a.n2max;
     const LoopOneLevel& L = a.lv[l];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int madeCount = a.meta[size_t(a.nl) * a.n2max * 4 + l];
     if (rank >= min(madeCount, a.n2max)) return;
     int32_t* meta = a.meta + (size_t(l) * a.n2max + rank) * 4;
@@ -879,44 +995,43 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter(LoopOneArgs a)
     int32_t* children = a.children + size_t(blockIdx.x) * a.childCap;
     if (threadIdx.x == 0) a.cflow[blockIdx.x] = L.flow[L.order[s]];
 
-    __shared__ int sNchild;
-
-    // children (Vote.cpp:396-412): voters of the points with >= voteMax/14 votes
-    if (warp == 0) {
-        int vmax = 1;
-        for (int k = lane; k < len; k += 32) vmax = max(vmax, voters(L, segc[-nf + k]));
-        for (int o = 16; o; o >>= 1) vmax = max(vmax, __shfl_xor_sync(kFull, vmax, o));
-        int nchild = 0;
-        for (int c0 = 0; c0 < len; c0 += 32) {
-            const int pos = c0 + lane;
-            const int e = pos < len ? segc[-nf + pos] : -1;
-            const int n = e >= 0 ? voters(L, e) : 0;
-            const int cnt = (n > 0 && n >= vmax / 14) ? n : 0;
-            int incl = cnt;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(kFull, incl, o);
-                if (lane >= o) incl += v;
-            }
-            const int excl = incl - cnt;
-            const int base = cnt ? L.voff[e] : 0;
-            const int tot = __shfl_sync(kFull, incl, 31);
-            // the chunk's voter lists, 32 entries at a time: entry o belongs to
-            // the first lane whose inclusive count exceeds o
-            for (int o0 = 0; o0 < tot; o0 += 32) {
-                const int o = o0 + lane;
-                int w = 0;
-                for (int b = 16; b > 0; b >>= 1)
-                    if (__shfl_sync(kFull, incl, w + b - 1) <= o) w += b;
-                const int wbase = __shfl_sync(kFull, base, w & 31);
-                const int wexcl = __shfl_sync(kFull, excl, w & 31);
-                if (o < tot && nchild + o < a.childCap) children[nchild + o] = L.vlist[wbase + (o - wexcl)];
-            }
-            nchild += tot;
+    // children (Vote.cpp:396-412): voters of the points with >= voteMax/14
+    // votes, in segment order: each thread takes two neighbouring points, and
+    // child o belongs to the last point whose offset is at most o
+    __shared__ int sWarp[32], sOff[2 * kFilterThreads], sBase[2 * kFilterThreads], sMax;
+    static_assert(kSegSlot <= 2 * kFilterThreads, "two points per thread");
+    if (tid == 0) sMax = 1;
+    __syncthreads();
+    int base[2] = {0, 0}, cnt[2] = {0, 0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        if (2 * tid + h < len) {
+            const int e = segc[-nf + 2 * tid + h];
+            base[h] = L.voff[e];
+            cnt[h] = L.voff[e + 1] - base[h];
         }
-        if (lane == 0) sNchild = nchild;
+    const int vmx = __reduce_max_sync(kFull, max(cnt[0], cnt[1]));
+    if (lane == 0) atomicMax(&sMax, vmx);
+    __syncthreads();
+    const int vmax = sMax;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        if (cnt[h] < vmax / 14) cnt[h] = 0;
+    int nchild;
+    const int incl = block_inclusive(cnt[0] + cnt[1], sWarp, nchild);
+    sOff[2 * tid] = incl - cnt[0] - cnt[1];
+    sOff[2 * tid + 1] = incl - cnt[1];
+    sBase[2 * tid] = base[0];
+    sBase[2 * tid + 1] = base[1];
+    __syncthreads();
+    for (int o = tid; o < min(nchild, a.childCap); o += kFilterThreads) {
+        int w = 0;
+#pragma unroll
+        for (int h = kFilterThreads; h > 0; h >>= 1)
+            if (sOff[w + h] <= o) w += h;
+        children[o] = L.vlist[sBase[w] + (o - sOff[w])];
     }
     __syncthreads();
-    const int nchild = sNchild;
     if (nchild > a.childCap) {
         if (tid == 0) {
             atomicOr(a.err, kLoopOneErrChildren);
@@ -984,51 +1099,23 @@ __device__ bool refit_row(const geo::Mat3& Qi, const geo::Mat3& Qo, int W, int y
     return true;
 }
 
-// Edge points of row y taken into the hull, in x order: written at out[]
-// when out is not null; returns their number.
-__device__ int refit_row_takes(const LoopOneLevel& L, const geo::Mat3& Qi, const geo::Mat3& Qo, float inCx,
-                               float inCy, int y, int32_t* out)
-{
-    int nr, xb[2], xe[2];
-    if (!refit_row(Qi, Qo, L.W, y, nr, xb, xe)) return 0;
-    int n = 0;
-    // the edge pixels of each x range, a bitmap word at a time, in x order
-    const uint2* row = L.bitidx + size_t(y) * L.WW;
-    for (int r = 0; r < nr; ++r) {
-        if (xb[r] > xe[r]) continue;
-        for (int wx = xb[r] >> 5; wx <= xe[r] >> 5; ++wx) {
-            const int lo = wx << 5;
-            const uint2 word = row[wx];
-            uint32_t w = word.x;
-            if (xb[r] > lo) w &= 0xffffffffu << (xb[r] - lo);
-            if (xe[r] < lo + 31) w &= 0xffffffffu >> (31 - (xe[r] - lo));
-            while (w) {
-                const int b = __ffs(w) - 1;
-                w &= w - 1;
-                const int e = int(word.y) + __popc(word.x & ((1u << b) - 1u));
-                if (e >= L.E) break;  // past a clamped edge count
-                const float cx = inCx - float(px_(L, e)), cy = inCy - float(py_(L, e));
-                if (gdx(L, e) * cx + gdy(L, e) * cy < 0) {
-                    if (out) out[n] = e;
-                    ++n;
-                }
-            }
-        }
-    }
-    return n;
-}
-
 // Multiresolution.cpp:319-401: level-0 hull of one coarse-level marker (rows
 // from the center row down the image until one misses the hull, then from
-// the center row up), then the outlier removal without weights.
-__global__ void __launch_bounds__(kFilterThreads) k_refit(LoopOneLevel L, const RefitTask* tasks, int32_t* hullAll,
-                                                        int hullCap, int32_t* rowsAll, int rowStride, int32_t* counts)
+// the center row up), one block per marker: 8 lanes per row, 128 rows at once,
+// each lane a contiguous part of the row's bitmap words, which it reads twice
+// (counting, then writing past a block scan of the counts: the second time
+// from L1), so that the points keep the order of rows and columns.
+// Measured (13 markers of a 1080p frame, cold): 18 us here and 46 us in the
+// outlier removal, 125 us with a thread per run of rows in the removal's block
+// of 128 threads (43 markers of a 3840x2160 clutter frame: 27 + 62 us, 188 us).
+constexpr int kHullThreads = 1024;
+constexpr int kHullLanes = 8;
+__global__ void __launch_bounds__(kHullThreads) k_refit_hull(LoopOneLevel L, const RefitTask* tasks, int32_t* hullAll,
+                                                             int hullCap, int32_t* counts)
 {
     const int b = blockIdx.x, tid = threadIdx.x;
     const RefitTask& T = tasks[b];
     int32_t* hull = hullAll + size_t(b) * hullCap;
-    int32_t* rowOff = rowsAll + size_t(b) * rowStride;
-    int32_t* err = counts + gridDim.x;
     geo::Mat3 Qi, Qo;
     for (int k = 0; k < 9; ++k) {
         Qi.m[k / 3][k % 3] = T.qin[k];
@@ -1036,65 +1123,80 @@ __global__ void __launch_bounds__(kFilterThreads) k_refit(LoopOneLevel L, const 
     }
     const int maxY = max(host_int(T.yc), 0);
     const int minY = min(host_int(T.yc), L.H - 1);
-    __shared__ int sUpEnd, sDownEnd, sTotal;
-    __shared__ int sPart[kFilterThreads];
+    __shared__ int sUpEnd, sDownEnd, sWarp[32];
     if (tid == 0) {
         sUpEnd = L.H;
         sDownEnd = -1;
     }
     __syncthreads();
     int nr, xb[2], xe[2];
-    for (int y = maxY + tid; y < L.H; y += blockDim.x)
+    for (int y = maxY + tid; y < L.H; y += kHullThreads)
         if (!refit_row(Qi, Qo, L.W, y, nr, xb, xe)) atomicMin(&sUpEnd, y);
-    for (int y = minY - tid; y >= 0; y -= blockDim.x)
+    for (int y = minY - tid; y >= 0; y -= kHullThreads)
         if (!refit_row(Qi, Qo, L.W, y, nr, xb, xe)) atomicMax(&sDownEnd, y);
     __syncthreads();
     const int rUp = max(sUpEnd - maxY, 0), rDown = max(minY - sDownEnd, 0);
     const int R = rUp + rDown;
-    auto row_y = [&](int r) { return r < rUp ? maxY + r : minY - (r - rUp); };
-    // per-row counts in processing order, contiguous chunks per thread
-    const int chunk = (R + blockDim.x - 1) / blockDim.x;
-    const int r0 = min(R, tid * chunk), r1 = min(R, r0 + chunk);
-    int part = 0;
-    for (int r = r0; r < r1; ++r) {
-        const int c = refit_row_takes(L, Qi, Qo, T.inCx, T.inCy, row_y(r), nullptr);
-        rowOff[r] = c;
-        part += c;
+    const int j = tid % kHullLanes;
+    int total = 0;
+    for (int r0 = 0; r0 < R; r0 += kHullThreads / kHullLanes) {
+        const int r = r0 + tid / kHullLanes;
+        const int y = r < rUp ? maxY + r : minY - (r - rUp);
+        // this lane's words [t0, t1) of the row's: w[0] words of the first x
+        // range, then those of the second
+        int w[2] = {0, 0}, t0 = 0, t1 = 0;
+        if (r < R && refit_row(Qi, Qo, L.W, y, nr, xb, xe)) {
+            for (int q = 0; q < nr; ++q)
+                if (xb[q] <= xe[q]) w[q] = (xe[q] >> 5) - (xb[q] >> 5) + 1;
+            const int per = (w[0] + w[1] + kHullLanes - 1) / kHullLanes;
+            t0 = min(j * per, w[0] + w[1]);
+            t1 = min(t0 + per, w[0] + w[1]);
+        }
+        // the edge points of those words that are taken into the hull, in x
+        // order; f(e) is called for each
+        auto each = [&](auto&& f) {
+            const uint2* row = L.bitidx + size_t(y) * L.WW;
+            for (int t = t0; t < t1; ++t) {
+                const int q = t < w[0] ? 0 : 1;
+                const int wx = (xb[q] >> 5) + t - (q ? w[0] : 0), lo = wx << 5;
+                const uint2 word = row[wx];
+                uint32_t m = word.x;
+                if (xb[q] > lo) m &= 0xffffffffu << (xb[q] - lo);
+                if (xe[q] < lo + 31) m &= 0xffffffffu >> (31 - (xe[q] - lo));
+                for (; m; m &= m - 1) {
+                    const int bit = __ffs(m) - 1;
+                    const int e = int(word.y) + __popc(word.x & ((1u << bit) - 1u));
+                    if (e >= L.E) break;  // past a clamped edge count
+                    const float cx = T.inCx - float(lo + bit), cy = T.inCy - float(y);
+                    if (gdx(L, e) * cx + gdy(L, e) * cy < 0) f(e);
+                }
+            }
+        };
+        int n = 0;
+        each([&](int) { ++n; });
+        int sum;
+        int off = total + block_inclusive(n, sWarp, sum) - n;
+        total += sum;
+        if (total <= hullCap)
+            each([&](int e) { hull[off++] = e; });
     }
-    sPart[tid] = part;
-    __syncthreads();
     if (tid == 0) {
-        int acc = 0;
-        for (int k = 0; k < int(blockDim.x); ++k) {
-            const int v = sPart[k];
-            sPart[k] = acc;
-            acc += v;
-        }
-        sTotal = acc;
+        if (total > hullCap) atomicOr(counts + gridDim.x, kLoopOneErrChildren);
+        counts[b] = total > hullCap || total < 5 ? -1 : total;
     }
-    __syncthreads();
-    const int total = sTotal;
-    if (total > hullCap) {
-        if (tid == 0) {
-            atomicOr(err, kLoopOneErrChildren);
-            counts[b] = -1;
-        }
-        return;
-    }
-    int off = sPart[tid];
-    for (int r = r0; r < r1; ++r) {
-        const int c = rowOff[r];
-        refit_row_takes(L, Qi, Qo, T.inCx, T.inCy, row_y(r), hull + off);
-        off += c;
-    }
-    __syncthreads();
-    if (total < 5) {
-        if (tid == 0) counts[b] = -1;
-        return;
-    }
-    const geo::Pcg32 rng(271828, (uint64_t(1) << 62) | uint64_t(T.marker));
-    const int nflt = lmeds_outliers(L, hull, total, false, 20.0f, rng, err);
-    if (tid == 0) counts[b] = nflt;
+}
+
+// ... then the outlier removal without weights.
+__global__ void __launch_bounds__(kFilterThreads) k_refit(LoopOneLevel L, const RefitTask* tasks, int32_t* hullAll,
+                                                        int hullCap, int32_t* counts)
+{
+    const int b = blockIdx.x;
+    const int total = counts[b];
+    if (total < 5) return;
+    const geo::Pcg32 rng(271828, (uint64_t(1) << 62) | uint64_t(tasks[b].marker));
+    const int nflt =
+        lmeds_outliers(L, hullAll + size_t(b) * hullCap, total, false, 20.0f, rng, counts + gridDim.x);
+    if (threadIdx.x == 0) counts[b] = nflt;
 }
 
 __global__ void __launch_bounds__(256) k_refit_pack(const int32_t* hullAll, int hullCap, const int32_t* counts,
@@ -1243,8 +1345,7 @@ LoopOneGpu::~LoopOneGpu()
     for (void* q : allocs_) cudaFree(q);
     if (args_.children) cudaFree(args_.children);
     if (d_packed_) cudaFree(d_packed_);
-    for (void* q : {static_cast<void*>(d_rtask_), static_cast<void*>(d_rhull_), static_cast<void*>(d_rrows_),
-                    static_cast<void*>(d_rcount_), static_cast<void*>(d_rpacked_)})
+    for (void* q : {static_cast<void*>(d_rtask_), static_cast<void*>(d_rhull_), static_cast<void*>(d_rcount_), static_cast<void*>(d_rpacked_)})
         if (q) cudaFree(q);
     if (h_rtask_) cudaFreeHost(h_rtask_);
     if (h_rcount_) cudaFreeHost(h_rcount_);
@@ -1434,20 +1535,18 @@ void LoopOneGpu::collect(cudaStream_t s, std::vector<LoopTwoIn>& out)
 void LoopOneGpu::ensure_refit_capacity(int n)
 {
     if (n <= refitCap_) return;
-    for (void* q : {static_cast<void*>(d_rtask_), static_cast<void*>(d_rhull_), static_cast<void*>(d_rrows_),
-                    static_cast<void*>(d_rcount_), static_cast<void*>(d_rpacked_)})
+    for (void* q : {static_cast<void*>(d_rtask_), static_cast<void*>(d_rhull_), static_cast<void*>(d_rcount_), static_cast<void*>(d_rpacked_)})
         if (q) cudaFree(q);
     if (h_rtask_) cudaFreeHost(h_rtask_);
     if (h_rcount_) cudaFreeHost(h_rcount_);
     d_rtask_ = nullptr;
-    d_rhull_ = d_rrows_ = d_rcount_ = d_rpacked_ = nullptr;
+    d_rhull_ = d_rcount_ = d_rpacked_ = nullptr;
     h_rtask_ = nullptr;
     h_rcount_ = nullptr;
     refitCap_ = 0;
     const int cap = std::max(n, 64);
     CCTAGB_CUDA(cudaMalloc(&d_rtask_, sizeof(RefitTask) * cap));
     CCTAGB_CUDA(cudaMalloc(&d_rhull_, sizeof(int32_t) * size_t(cap) * hullCap_));
-    CCTAGB_CUDA(cudaMalloc(&d_rrows_, sizeof(int32_t) * size_t(cap) * (maxH_ + 2)));
     CCTAGB_CUDA(cudaMalloc(&d_rcount_, sizeof(int32_t) * (cap + 1)));
     CCTAGB_CUDA(cudaMalloc(&d_rpacked_, sizeof(int32_t) * size_t(cap) * hullCap_));
     CCTAGB_CUDA(cudaMallocHost(&h_rtask_, sizeof(RefitTask) * cap));
@@ -1471,7 +1570,9 @@ void LoopOneGpu::refit(const Levels& lv, const std::vector<RefitTask>& tasks, cu
     const size_t hullMax = size_t(L.E) + size_t(L.W) + 1;
     for (;;) {
         CCTAGB_CUDA(cudaMemsetAsync(d_rcount_ + n, 0, sizeof(int32_t), s));
-        k_refit<<<n, kFilterThreads, 0, s>>>(L, d_rtask_, d_rhull_, hullCap_, d_rrows_, maxH_ + 2, d_rcount_);
+        k_refit_hull<<<n, kHullThreads, 0, s>>>(L, d_rtask_, d_rhull_, hullCap_, d_rcount_);
+        CCTAGB_CUDA(cudaGetLastError());
+        k_refit<<<n, kFilterThreads, 0, s>>>(L, d_rtask_, d_rhull_, hullCap_, d_rcount_);
         CCTAGB_CUDA(cudaGetLastError());
         k_refit_pack<<<n, 256, 0, s>>>(d_rhull_, hullCap_, d_rcount_, d_rpacked_);
         CCTAGB_CUDA(cudaGetLastError());

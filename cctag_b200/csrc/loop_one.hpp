@@ -98,7 +98,7 @@ public:
     void refit(const Levels& lv, const std::vector<RefitTask>& tasks, cudaStream_t s,
                std::vector<std::vector<int32_t>>& filtered);
     int launches() const { return 6 + chainLaunches_; }
-    int refit_launches() const { return 2; }
+    int refit_launches() const { return 3; }
     long long h2d_bytes() const { return h2d_; }
     long long d2h_bytes() const { return d2h_; }
 
@@ -124,7 +124,6 @@ private:
     RefitTask* h_rtask_ = nullptr;
     int hullCap_ = kChildCap;       // room for one marker's hull points
     int32_t* d_rhull_ = nullptr;    // refitCap_ * hullCap_
-    int32_t* d_rrows_ = nullptr;    // refitCap_ * (maxH_ + 2) per-row offsets
     int32_t* d_rcount_ = nullptr;   // refitCap_ + 1 (last: error bits)
     int32_t* h_rcount_ = nullptr;
     int32_t* d_rpacked_ = nullptr;  // refitCap_ * hullCap_
