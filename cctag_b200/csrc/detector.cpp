@@ -122,15 +122,35 @@ void Detector::identify_on(const uint8_t* d_img, size_t pitch, const IdentTask* 
     if (n <= 0) return;
     if (bank_.empty()) throw Error{CCTAGB_BANK_ERROR, "no marker bank for this number of crowns"};
     ensure_ident_capacity(n);
-    std::memcpy(h_tasks_, tasks, sizeof(IdentTask) * n);
+    // Largest ellipses first: they take the most rounds and the longest reads,
+    // and a block that starts one last leaves the other SMs idle (1024 grid
+    // candidates: 1.48 ms, 1.95 ms in the caller's order).  A counting sort by
+    // the exponent and two mantissa bits of the larger axis.
+    auto size_key = [](const IdentTask& t) {
+        const float m = std::max(std::fabs(t.a), std::fabs(t.b));
+        uint32_t bits;
+        std::memcpy(&bits, &m, sizeof(bits));
+        return 1023u - (bits >> 21);
+    };
+    int first[1025] = {};
+    for (int i = 0; i < n; ++i) ++first[size_key(tasks[i]) + 1];
+    for (int k = 0; k < 1024; ++k) first[k + 1] += first[k];
+    ident_order_.resize(size_t(n));
+    for (int i = 0; i < n; ++i) ident_order_[size_t(first[size_key(tasks[i])]++)] = i;
+    for (int i = 0; i < n; ++i) h_tasks_[i] = tasks[ident_order_[size_t(i)]];
     cudaStream_t s = pipe_.stream();
     CCTAGB_CUDA(cudaMemcpyAsync(d_tasks_, h_tasks_, sizeof(IdentTask) * n, cudaMemcpyHostToDevice, s));
     CCTAGB_CUDA(cudaEventRecord(ev_id0_, s));
-    launch_identify(d_img, pitch, d_tasks_, d_res_, n, d_bank_inv_, ip, s);
+    int maxCuts = 1, maxBox = 0;
+    for (int i = 0; i < n; ++i) {
+        maxCuts = std::max(maxCuts, tasks[i].ncuts);
+        maxBox = std::max(maxBox, ident_box(tasks[i].a, tasks[i].b, tasks[i].angle));
+    }
+    launch_identify(d_img, pitch, d_tasks_, d_res_, n, maxCuts, maxBox, d_bank_inv_, ip, s);
     CCTAGB_CUDA(cudaEventRecord(ev_id1_, s));
     CCTAGB_CUDA(cudaMemcpyAsync(h_res_, d_res_, sizeof(IdentResult) * n, cudaMemcpyDeviceToHost, s));
     pipe_.host_wait(s);
-    std::memcpy(out, h_res_, sizeof(IdentResult) * n);
+    for (int i = 0; i < n; ++i) out[ident_order_[size_t(i)]] = h_res_[i];
     pipe_.add_io((long long)sizeof(IdentTask) * n, (long long)sizeof(IdentResult) * n, 1);
 }
 
@@ -189,7 +209,10 @@ void Detector::select_and_identify(int nm, int npts, int w, int h)
     launch_outer_select(d_cutin_, d_cutpts_, cp.nOuter, d_sel_, d_nsel_, nm, s);
     launch_cut_select(pipe_.level0_src(), w, h, d_cutin_, d_cutpts_, d_sel_, d_nsel_, d_tasks_, d_st1_, nm, cp, s);
     CCTAGB_CUDA(cudaEventRecord(ev_id0_, s));
-    launch_identify(pipe_.level0_src(), size_t(w), d_tasks_, d_res_, nm, d_bank_inv_,
+    int maxBox = 0;
+    for (int i = 0; i < nm; ++i)
+        maxBox = std::max(maxBox, ident_box(h_tasks_[i].a, h_tasks_[i].b, h_tasks_[i].angle));
+    launch_identify(pipe_.level0_src(), size_t(w), d_tasks_, d_res_, nm, cp.maxSelect, maxBox, d_bank_inv_,
                     ident_params(params_.refineMode), s);
     CCTAGB_CUDA(cudaEventRecord(ev_id1_, s));
     CCTAGB_CUDA(cudaMemcpyAsync(h_res_, d_res_, sizeof(IdentResult) * nm, cudaMemcpyDeviceToHost, s));

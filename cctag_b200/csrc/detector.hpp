@@ -92,6 +92,7 @@ private:
     IdentTask* h_tasks_ = nullptr;
     IdentResult* h_res_ = nullptr;
     int ident_cap_ = 0;
+    std::vector<int> ident_order_;               // identify_on: the caller's task of each launched one
     float* d_centers_ = nullptr;
     float* d_cost_ = nullptr;
     float* h_cost_ = nullptr;

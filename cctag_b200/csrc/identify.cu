@@ -1,13 +1,13 @@
-// Identification on sm_100a: imaged-center refinement and ID reading, one
-// thread block per marker (Identification.cpp:813-1158 refineConicFamilyGlob /
-// imageCenterOptimizationGlob / costFunctionGlob / getSignals, and
-// :50-193 orazioDistanceRobust, :1408-1436 ID vote).
+// Identification on sm_100a: imaged-center refinement and ID reading, a thread
+// block or a cluster of them per marker (Identification.cpp:813-1158
+// refineConicFamilyGlob / imageCenterOptimizationGlob / costFunctionGlob /
+// getSignals, and :50-193 orazioDistanceRobust, :1408-1436 ID vote).
 //
 // Grid refinement: each round evaluates a gridN x gridN set of trial centres
-// (getNearbyPoints, conditioned by the ellipse) with one warp per trial.  A
-// trial's homography maps the unit circle to the outer ellipse and the origin
-// to the trial centre (computeHomographyFromEllipseAndImagedCenter); every cut
-// is resampled in the marker plane along the ray to its back-projected end.
+// (getNearbyPoints, conditioned by the ellipse).  A trial's homography maps the
+// unit circle to the outer ellipse and the origin to the trial centre
+// (computeHomographyFromEllipseAndImagedCenter); every cut is resampled in the
+// marker plane along the ray to its back-projected end.
 //
 // The reference marks a cut "out of bounds" the first time any of its samples
 // leaves the image, for every later trial and round (the flag lives in the cut
@@ -19,9 +19,20 @@
 // Cost: the reference's mean over cut pairs of sum_k (s_i[k] - s_j[k])^2, here
 // in the equivalent form n * sum_i (s_i[k] - mean_k)^2 summed over k, divided
 // by the n(n-1)/2 pairs (shifted FP32 sums per sample, FP64 over samples).
-// The sample loop avoids the XU pipe (conversions, divisions), which bounds
-// a straightforward version of it.
+//
+// The kernel is bound by instruction issue and by the reads of the samples: a
+// 22-cut, 100-sample, 25-trial round is 55,000 bilinear samples, whose lanes lie
+// along a ray and so on many lines of the L1 (read from the image, four bytes
+// each, they kept it 90 % busy).  So the marker's pixels are staged in shared
+// memory, with rows an odd number of words apart; the sample loop is kept to
+// some 45 instructions a sample (no IEEE division, the clamp and the integer
+// part of a coordinate in one operation, constant factors left to the end); no
+// lane idles on the samples past a multiple of 32 (they are packed several
+// trials to a warp); and the serial parts (statistics of a signal, medians, the
+// distances to the bank) are spread over lanes, warps and blocks.
+#include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <cstdint>
 
 #include <cooperative_groups.h>
@@ -35,17 +46,16 @@ namespace cctagb {
 namespace {
 
 constexpr int kMaxTrials = 25;
-constexpr int kThreads = 32 * kMaxTrials;
+constexpr int kThreads = 32 * kMaxTrials;  // of the cost kernels
 constexpr int kWarps = kThreads / 32;
-// The samples along a cut come in chunks of 32 (one per lane).  A marker is
-// either one thread block doing every chunk, or a cluster of kCluster blocks,
-// block r doing chunk r, whose per-chunk sums meet through distributed shared
-// memory: few markers per launch spread over four SMs each, many markers
-// keep one SM each.  Per-chunk sums are formed the same way in both, and
-// added in chunk order, so both give the same bits.
+// The samples along a cut come in chunks of 32 (one per lane).  Per-chunk sums
+// are formed the same way in every block layout and added in chunk order, so
+// all layouts give the same bits.
 constexpr int kChunk = 32;
 constexpr int kMaxChunks = kMaxSamples / kChunk;
-constexpr int kCluster = kMaxChunks;
+constexpr int kMaxCluster = 8;      // blocks per marker at most
+constexpr int kMaxIdWarps = 20;     // warps per block of k_identify at most
+constexpr int kGnBlocks = 7;        // blocks per SM of a large Gauss-Newton launch
 
 __device__ __forceinline__ void mat_mul(const float* a, const float* b, float* r)
 {
@@ -188,6 +198,43 @@ __device__ void homography_from_center(const float* C, const float* Tp, const fl
     mat_mul(Td, h, H);
 }
 
+// The image of a cut's samples under a trial homography: sample k is at
+// (U0 + k dU, V0 + k dV) / (W0 + k dW).  One entry of padding per trial keeps
+// lanes that read different trials on different banks.
+struct TrialLines {
+    float4* uv;  // U0 dU V0 dV, entry t * stride + cut
+    float2* w;   // W0 dW
+    int stride;
+};
+__device__ __forceinline__ TrialLines trial_lines(void* work, int trials, int ncuts)
+{
+    float4* uv = static_cast<float4*>(work);
+    return TrialLines{uv, reinterpret_cast<float2*>(uv + trials * (ncuts + 1)), ncuts + 1};
+}
+struct GnChunk {  // Gauss-Newton, one chunk of samples
+    float s[kMaxCuts][kChunk];            // value
+    float dx[kMaxCuts][kChunk];           // d value / d center x
+    float dy[kMaxCuts][kChunk];           // d value / d center y
+};
+constexpr int kGnWhole = 2400;            // cuts x samples whose values and derivatives fit at once
+constexpr int kSigStride = kMaxSamples + 1;
+// What the reading of the cuts keeps once the center is found.
+struct FinalWork {
+    float sig[kMaxCuts][kSigStride];                // final signals
+    uint32_t black[kMaxBankIds][kMaxSamples / 32];  // per bank row: samples inside an odd number of its rings
+    float barcode[kMaxSamples];
+};
+// Dynamic shared memory: the lines of the grid rounds (an entry of padding past
+// the cuts) or Gauss-Newton's samples, then the marker's pixels; at the end
+// FinalWork in their place.
+__host__ __device__ constexpr size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
+__host__ __device__ constexpr size_t grid_work(int trials, int ncuts)
+{
+    return align16(size_t(trials) * (ncuts + 1) * (sizeof(float4) + sizeof(float2)));
+}
+constexpr size_t kGnWork = 3 * sizeof(float) * kGnWhole;
+static_assert(sizeof(GnChunk) <= kGnWork, "the chunk form fits");
+
 struct Shared {
     float C[9], Tp[9], Td[9];
     float mT[9], mTi[9];
@@ -198,74 +245,153 @@ struct Shared {
     uint32_t oob;                  // sticky out-of-bounds cut mask
     int rounds;
     int fail;
-    float trialH[kMaxTrials][9];
+    float trialH[kMaxTrials][9], trialHi[kMaxTrials][9];
+    int trialOk[kMaxTrials];       // the homography has an inverse
     float trialPt[kMaxTrials][2];
-    union {
-        float cutp[kMaxTrials][kMaxCuts][6];  // grid: image line of the cut's samples, U0 dU V0 dV W0 dW
-        struct {                              // Gauss-Newton: one chunk of samples
-            float s[kMaxCuts][kChunk];        // value
-            float dx[kMaxCuts][kChunk];       // d value / d center x
-            float dy[kMaxCuts][kChunk];       // d value / d center y
-        } gn;
-    } u;
     // Gauss-Newton state
     float gH[9], gHi[9], gdH[2][9], gdHi[2][9];  // homography at the trial center, inverse, center derivatives
     float gTry[2];                               // trial center
     uint32_t gOob;                               // cuts whose end samples leave the rectangle at the trial
+    float gBack[kMaxCuts][6];                    // back-projected cut ends and their center derivatives
     double gPart[2][kMaxChunks][6];              // per-chunk sums (cost, J^T r, J^T J) by parity
     double gSum[6];
     double gA[3], gG[2], gBest, gLambda;         // normal equations at the best center, its cost, damping
     int gHave, gStop, iterations;
     uint32_t trialOob[kMaxTrials];
-    uint32_t valid[kMaxTrials];
-    float cost[kMaxTrials];
+    int box[4];                              // the staged pixels' rectangle x0 y0 x1 y1 (empty: none), as roi
+    int direct;                              // a sample of the round lies outside them
     double part[2][kMaxChunks][kMaxTrials];  // per-chunk shares of each trial's cost (by round parity)
-    float sig[kMaxCuts][kMaxSamples];
-    float barcode[kMaxSamples];
+    float radius[kMaxSamples];               // the samples' plane radii
+    float rcp[kMaxSamples + 1];              // 1 / i, rounded
+    float stats[kMaxCuts][4];                // of a cut's signal: black and white mean, 1 / (2 variance) (a double)
     int winner[kMaxCuts];
     float vwin[kMaxCuts];
 };
 
-// Per trial (one warp): homography, the image line of each cut's samples and
-// the cuts whose end samples leave the rectangle.
-__device__ void setup_trial(Shared& S, const IdentTask& T, int t, float px, float py, const IdentParams& ip,
-                            const Roi& R, int lane)
+// 1 / w without the fix-up for denormals and the largest floats, which a
+// homography's scale does not reach.
+__device__ __forceinline__ float fast_rcp(float w)
 {
-    float Hm[9], Hi[9];
-    homography_from_center(S.C, S.Tp, S.Td, px, py, Hm);
-    const bool ok = mat_inv(Hm, Hi);
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) S.trialH[t][k] = Hm[k];
-        S.trialPt[t][0] = px;
-        S.trialPt[t][1] = py;
-    }
-    bool bad = false;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(w));
+    return r;
+}
+
+// Whether a sample's pixels are staged: a pixel's distance from the edges of
+// the staged rectangle, for the rounding of samples between two such ends (at
+// an edge that is the candidate's rectangle's own, as that is read).
+__device__ __forceinline__ bool in_box(const Shared& S, const Roi& R, float x, float y)
+{
+    return x >= float(S.box[0] + (S.box[0] > R.x0 ? 1 : 0)) && x < float(S.box[2] - (S.box[2] < R.x1 ? 2 : 1)) &&
+           y >= float(S.box[1] + (S.box[1] > R.y0 ? 1 : 0)) && y < float(S.box[3] - (S.box[3] < R.y1 ? 2 : 1));
+}
+
+// Bytes per row of the staged pixels: an odd number of words, so that a column
+// of them spreads over all banks.
+__device__ __forceinline__ int box_pitch(const Shared& S) { return (((S.box[2] - S.box[0] + 3) >> 2) | 1) << 2; }
+
+// The rectangle that holds the marker's samples with their neighbours (the
+// segments from the cut ends to near the center), clipped to the candidate's
+// rectangle; empty when it takes more than `room` bytes.  By a warp.
+__device__ void find_box(Shared& S, const IdentTask& T, const Roi& R, size_t room, int lane)
+{
+    float x = T.x0, y = T.y0;
     if (lane < T.ncuts) {
-        float bx, by, w;
-        if (ok) apply_h(Hi, T.stop[lane][0], T.stop[lane][1], bx, by, w);
-        else bx = by = NAN;
-        const float xs = bx * ip.beginSig, ys = by * ip.beginSig;
-        const float sx = (bx - xs) / (float(ip.nSamples) - 1.f), sy = (by - ys) / (float(ip.nSamples) - 1.f);
-        // sample k is (xs + k sx, ys + k sy) in the marker plane; its image in
-        // homogeneous coordinates is linear in k: H (xs, ys, 1) + k H (sx, sy, 0)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            S.u.cutp[t][lane][2 * i] = __fmaf_rn(Hm[3 * i], xs, __fmaf_rn(Hm[3 * i + 1], ys, Hm[3 * i + 2]));
-            S.u.cutp[t][lane][2 * i + 1] = __fmaf_rn(Hm[3 * i], sx, __fmul_rn(Hm[3 * i + 1], sy));
-        }
-        // end samples, with the sample loop's own arithmetic
-        const float* cp = S.u.cutp[t][lane];
-        const float kl = float(ip.nSamples - 1);
-        const float w0 = cp[4], w1 = __fmaf_rn(kl, cp[5], cp[4]);
-        const float r0 = __fdividef(1.0f, w0), r1 = __fdividef(1.0f, w1);
-        const float x0 = __fmul_rn(cp[0], r0), y0 = __fmul_rn(cp[2], r0);
-        const float x1 = __fmul_rn(__fmaf_rn(kl, cp[1], cp[0]), r1), y1 = __fmul_rn(__fmaf_rn(kl, cp[3], cp[2]), r1);
-        bad = !(w0 > 0.f && w1 > 0.f) && !(w0 < 0.f && w1 < 0.f);
-        bad = bad || !inside(R, x0, y0) || !inside(R, x1, y1);
+        x = T.stop[lane][0];
+        y = T.stop[lane][1];
     }
-    const uint32_t m = __ballot_sync(0xffffffffu, bad);
-    if (lane == 0) S.trialOob[t] = m & ((T.ncuts >= 32) ? 0xffffffffu : ((1u << T.ncuts) - 1u));
+    float x0 = fminf(x, T.x0), x1 = fmaxf(x, T.x0), y0 = fminf(y, T.y0), y1 = fmaxf(y, T.y0);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+        y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
+        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+        y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+    }
+    if (lane == 0) {
+        // finite (checked by the host, or refined image points); clipped as
+        // floats first, so that the conversions are in range
+        S.box[0] = int(fminf(fmaxf(x0 - 2.f, float(R.x0)), float(R.x1)));
+        S.box[1] = int(fminf(fmaxf(y0 - 2.f, float(R.y0)), float(R.y1)));
+        S.box[2] = int(fminf(fmaxf(x1 + 4.f, float(R.x0)), float(R.x1)));
+        S.box[3] = int(fminf(fmaxf(y1 + 4.f, float(R.y0)), float(R.y1)));
+        // a row start on a word boundary, where the image's rows are
+        const int down = int(reinterpret_cast<size_t>(R.img + S.box[0]) & 3);
+        if (R.pitch % 4 == 0 && S.box[0] - down >= R.x0) S.box[0] -= down;
+        const int w = S.box[2] - S.box[0], h = S.box[3] - S.box[1];
+        if (w < 4 || h < 4 || size_t(box_pitch(S)) * size_t(h) > room)
+            S.box[0] = S.box[1] = S.box[2] = S.box[3] = 0;
+    }
+}
+
+// The pixels of the box into shared memory, a word of four at a time: a word
+// on a boundary by an asynchronous copy, another one put together from the two
+// it straddles (inside the row only), the ends of a row byte by byte.  The
+// caller's next barrier must follow cp.async.wait_all of every thread.
+__device__ void stage_box(const Shared& S, const Roi& R, uint8_t* px)
+{
+    const int w = S.box[2] - S.box[0], h = S.box[3] - S.box[1];
+    if (w <= 0) return;
+    const int pitch = box_pitch(S), words = (w + 3) >> 2;
+    const int nwarps = blockDim.x >> 5, lane = threadIdx.x & 31;
+    for (int y = threadIdx.x >> 5; y < h; y += nwarps) {
+        const uint8_t* row = R.img + size_t(S.box[1] + y) * R.pitch + size_t(S.box[0]);
+        const int shift = int(reinterpret_cast<size_t>(row) & 3);
+        uint32_t* out = reinterpret_cast<uint32_t*>(px + size_t(y) * pitch);
+#pragma unroll 4
+        for (int j = lane; j < words; j += 32) {
+            const uint8_t* p = row + 4 * j;
+            if (shift == 0 && 4 * j + 4 <= w) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                 unsigned(__cvta_generic_to_shared(out + j))),
+                             "l"(p)
+                             : "memory");
+                continue;
+            }
+            uint32_t v;
+            if (shift != 0 && j > 0 && 4 * j + 8 <= w) {
+                const uint32_t* q = reinterpret_cast<const uint32_t*>(p - shift);
+                v = __funnelshift_r(__ldg(q), __ldg(q + 1), 8 * shift);
+            } else {
+                v = 0u;
+                for (int k = 0; k < 4 && 4 * j + k < w; ++k) v |= uint32_t(__ldg(p + k)) << (8 * k);
+            }
+            out[j] = v;
+        }
+    }
+}
+
+// The image line of cut c under trial t's homography, and whether its end
+// samples leave the rectangle.
+__device__ __forceinline__ void setup_cut(Shared& S, const TrialLines& lines, const IdentTask& T, int t, int c,
+                                          const IdentParams& ip, const Roi& R)
+{
+    const float* Hm = S.trialH[t];
+    float bx, by, w;
+    if (S.trialOk[t]) apply_h(S.trialHi[t], T.stop[c][0], T.stop[c][1], bx, by, w);
+    else bx = by = NAN;
+    const float xs = bx * ip.beginSig, ys = by * ip.beginSig;
+    const float sx = (bx - xs) / (float(ip.nSamples) - 1.f), sy = (by - ys) / (float(ip.nSamples) - 1.f);
+    // sample k is (xs + k sx, ys + k sy) in the marker plane; its image in
+    // homogeneous coordinates is linear in k: H (xs, ys, 1) + k H (sx, sy, 0)
+    float cp[6];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        cp[2 * i] = __fmaf_rn(Hm[3 * i], xs, __fmaf_rn(Hm[3 * i + 1], ys, Hm[3 * i + 2]));
+        cp[2 * i + 1] = __fmaf_rn(Hm[3 * i], sx, __fmul_rn(Hm[3 * i + 1], sy));
+    }
+    lines.uv[t * lines.stride + c] = make_float4(cp[0], cp[1], cp[2], cp[3]);
+    lines.w[t * lines.stride + c] = make_float2(cp[4], cp[5]);
+    // end samples, with the sample loop's own arithmetic
+    const float kl = float(ip.nSamples - 1);
+    const float w0 = cp[4], w1 = __fmaf_rn(kl, cp[5], cp[4]);
+    const float r0 = fast_rcp(w0), r1 = fast_rcp(w1);
+    const float x0 = __fmul_rn(cp[0], r0), y0 = __fmul_rn(cp[2], r0);
+    const float x1 = __fmul_rn(__fmaf_rn(kl, cp[1], cp[0]), r1), y1 = __fmul_rn(__fmaf_rn(kl, cp[3], cp[2]), r1);
+    bool bad = !(w0 > 0.f && w1 > 0.f) && !(w0 < 0.f && w1 < 0.f);
+    bad = bad || !inside(R, x0, y0) || !inside(R, x1, y1);
+    if (bad) atomicOr(&S.trialOob[t], 1u << c);
+    else if (!(in_box(S, R, x0, y0) && in_box(S, R, x1, y1))) S.direct = 1;
 }
 
 // Byte -> float without a conversion instruction (exponent 2^23 trick).
@@ -312,23 +438,20 @@ __device__ __forceinline__ float bilinear_value(const float p[4], float fx, floa
     return __fmul_rn(a, 0.5f);
 }
 
-__device__ __forceinline__ float bilinear_in(const Roi& R, float x, float y)
-{
-    float p[4], fx, fy;
-    bilinear_taps(R, x, y, p, fx, fy);
-    return bilinear_value(p, fx, fy);
-}
-
 // Same value and its gradient in x and y (the derivative of the bilinear
 // patch the sample falls in).
-__device__ __forceinline__ float bilinear_grad(const Roi& R, float x, float y, float& gx, float& gy)
+__device__ __forceinline__ float bilinear_value_grad(const float p[4], float fx, float fy, float& gx, float& gy)
 {
-    float p[4], fx, fy;
-    bilinear_taps(R, x, y, p, fx, fy);
     const float fx1 = 1.0f - fx, fy1 = 1.0f - fy;
     gx = ((p[1] - p[0]) * fy1 + (p[3] - p[2]) * fy) * 0.5f;
     gy = ((p[2] - p[0]) * fx1 + (p[3] - p[1]) * fx) * 0.5f;
     return bilinear_value(p, fx, fy);
+}
+__device__ __forceinline__ float bilinear_grad(const Roi& R, float x, float y, float& gx, float& gy)
+{
+    float p[4], fx, fy;
+    bilinear_taps(R, x, y, p, fx, fy);
+    return bilinear_value_grad(p, fx, fy, gx, gy);
 }
 
 // Row i of H applied to (x, y, 1), explicit roundings.
@@ -337,17 +460,77 @@ __device__ __forceinline__ float hrow(const float* Hm, int i, float x, float y)
     return __fmaf_rn(Hm[3 * i], x, __fmaf_rn(Hm[3 * i + 1], y, Hm[3 * i + 2]));
 }
 
-// One sample of cut c of trial t: its point on the cut's image line, then a
-// bilinear read (fast reciprocal: one MUFU op, no IEEE fix-up).
-__device__ __forceinline__ float cut_sample(const Shared& S, const Roi& R, int t, int c, float kf)
+// The pixels as the sample loop reads them, from the image or staged: the
+// first pixel, and what turns the integer part of a coordinate (in the mantissa
+// of x + 2^23) into a pixel's index, clamped so that rounding at the border
+// never reads outside.
+template <bool STAGED>
+struct SampleArea {
+    const uint8_t* corner;
+    size_t pitch;
+    int biasX, biasY, maxX, maxY;
+};
+__device__ __forceinline__ SampleArea<false> image_area(const Roi& R)
 {
-    const float* cp = S.u.cutp[t][c];
-    const float u = __fmaf_rn(kf, cp[1], cp[0]);
-    const float v = __fmaf_rn(kf, cp[3], cp[2]);
-    const float w = __fmaf_rn(kf, cp[5], cp[4]);
-    const float r = __fdividef(1.0f, w);
-    return bilinear_in(R, __fmul_rn(u, r), __fmul_rn(v, r));
+    return {R.img + size_t(R.y0) * R.pitch + size_t(R.x0), R.pitch, -0x4B000000 - R.x0, -0x4B000000 - R.y0,
+            R.x1 - R.x0 - 2, R.y1 - R.y0 - 2};
 }
+__device__ __forceinline__ SampleArea<true> staged_area(const Shared& S, const uint8_t* px)
+{
+    return {px, size_t(box_pitch(S)), -0x4B000000 - S.box[0], -0x4B000000 - S.box[1], S.box[2] - S.box[0] - 2,
+            S.box[3] - S.box[1] - 2};
+}
+
+// The four pixels around (x, y), zero-extended, and the fractional offsets.
+template <bool STAGED>
+__device__ __forceinline__ void area_taps(const SampleArea<STAGED>& A, float x, float y, uint32_t p[4], float& fx,
+                                          float& fy)
+{
+    const float tx = __fadd_rz(fmaxf(x, 0.f), 8388608.f), ty = __fadd_rz(fmaxf(y, 0.f), 8388608.f);
+    fx = __fsub_rn(x, __fsub_rn(tx, 8388608.f));
+    fy = __fsub_rn(y, __fsub_rn(ty, 8388608.f));
+    const int px = __viaddmin_s32_relu(__float_as_int(tx), A.biasX, A.maxX);
+    const int py = __viaddmin_s32_relu(__float_as_int(ty), A.biasY, A.maxY);
+    if (STAGED) {
+        const int pitch = int(A.pitch), at = py * pitch + px;
+        p[0] = A.corner[at];
+        p[1] = A.corner[at + 1];
+        p[2] = A.corner[at + pitch];
+        p[3] = A.corner[at + pitch + 1];
+    } else {
+        const uint8_t* p0 = A.corner + size_t(unsigned(py)) * A.pitch + unsigned(px);
+        const uint8_t* p1 = p0 + A.pitch;
+        p[0] = __ldg(p0);
+        p[1] = __ldg(p0 + 1);
+        p[2] = __ldg(p1);
+        p[3] = __ldg(p1 + 1);
+    }
+}
+
+// 2^-22 times the bilinear value (Identification.hpp:197-219) of a sample of a
+// cut: its point on the cut's image line, then the read.  The operations and
+// their roundings are those of bilinear_value on scaled pixels: a byte taken as
+// the bits of a float is its value times 2^-149, and one product brings it to
+// 2^-23 of the pixel, exactly; the factor and the value's 1/2 are powers of two
+// that trial sums carry to their end (kTermScale).
+template <bool STAGED>
+__device__ __forceinline__ float cut_sample(const SampleArea<STAGED>& A, const float4& l, const float2& lw, float kf)
+{
+    const float r = fast_rcp(__fmaf_rn(kf, lw.y, lw.x));
+    const float x = __fmul_rn(__fmaf_rn(kf, l.y, l.x), r), y = __fmul_rn(__fmaf_rn(kf, l.w, l.z), r);
+    uint32_t p[4];
+    float fx, fy;
+    area_taps(A, x, y, p, fx, fy);
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = __fmul_rn(__uint_as_float(p[q]), 0x1p126f);
+    const float fx1 = __fsub_rn(1.0f, fx), fy1 = __fsub_rn(1.0f, fy);
+    float a = __fmul_rn(v[0], __fmul_rn(fx1, fy1));
+    a = __fmaf_rn(v[1], __fmul_rn(fx, fy1), a);
+    a = __fmaf_rn(v[2], __fmul_rn(fx1, fy), a);
+    return __fmaf_rn(v[3], __fmul_rn(fx, fy), a);
+}
+constexpr double kTermScale = 0x1p44;  // (2^22)^2
 
 // Sum over the 32 lanes (the same butterfly, so the same bits, everywhere).
 __device__ __forceinline__ double lane_sum(double v)
@@ -357,69 +540,139 @@ __device__ __forceinline__ double lane_sum(double v)
     return v;
 }
 
-// Per-chunk shares of the cost of trial t (one warp): chunks j0 .. j0+NCH-1
-// (those below nch), lane = sample within the chunk, over the valid cuts in
-// order, a few cuts at a time so that their reads overlap.  Per sample the
-// cut values are shifted by the first valid cut's value before the FP32 sums
-// (the term n * sum(d^2) - (sum d)^2 does not change under a common shift,
-// and the shifted sums stay small); out[q] is the chunk's FP64 lane sum.
-template <int NCH>
-__device__ void trial_partial(const Shared& S, const Roi& R, int t, uint32_t valid, int j0, int nch, int nS,
-                              int lane, double out[NCH])
+// Share of a trial's cost of one whole chunk (a warp, lane = sample within the
+// chunk): over the valid cuts in order, a few at a time so that their reads
+// overlap.  Per sample the cut values are shifted by the first valid cut's
+// value before the FP32 sums (the term n * sum(d^2) - (sum d)^2 does not change
+// under a common shift, and the shifted sums stay small), then summed over the
+// lanes in FP64.
+template <bool STAGED>
+__device__ __forceinline__ double trial_chunk(const TrialLines& lines, const SampleArea<STAGED>& A, int t,
+                                              uint32_t valid, int k)
 {
-    constexpr int G = NCH == 1 ? 4 : 2;  // cuts per step
+    constexpr int G = 4;  // cuts per step
     const int n = __popc(valid);
-    float v0[NCH], s1[NCH], s2[NCH], kf[NCH];
-    bool act[NCH];
-#pragma unroll
-    for (int q = 0; q < NCH; ++q) {
-        const int k = (j0 + q) * kChunk + lane;
-        act[q] = j0 + q < nch && k < nS;
-        // lanes past the last sample read the last one again (in bounds, no
-        // branch) and their terms are dropped below
-        kf[q] = float(min(k, nS - 1));
-        v0[q] = s1[q] = s2[q] = 0.f;
-    }
+    float v0 = 0.f, s1 = 0.f, s2 = 0.f;
+    const float kf = float(k);
     if (n >= 2) {
-        uint32_t m = valid;
-        bool first = true;  // the same in every lane: a uniform branch
-        while (m) {
-            int c[G];
-            float keep[G];
+        bool first = true;  // the same in every lane, as valid: uniform branches
+        for (uint32_t m = valid; m;) {
+            const int have = __popc(m);
+            float val[G];
 #pragma unroll
             for (int g = 0; g < G; ++g) {
-                // past the last valid cut: repeat it, with weight 0
-                c[g] = m ? __ffs(m) - 1 : c[g > 0 ? g - 1 : 0];
-                keep[g] = m ? 1.f : 0.f;
+                const int i = t * lines.stride + (m ? __ffs(m) - 1 : 0);  // past the last valid cut: read, not used
                 m &= m - 1;
+                val[g] = cut_sample(A, lines.uv[i], lines.w[i], kf);
             }
-            float val[G][NCH];
-#pragma unroll
-            for (int g = 0; g < G; ++g)
-#pragma unroll
-                for (int q = 0; q < NCH; ++q) val[g][q] = cut_sample(S, R, t, c[g], kf[q]);
-            if (first) {
-#pragma unroll
-                for (int q = 0; q < NCH; ++q) v0[q] = val[0][q];  // first valid cut: the shift
-                first = false;
-            }
+            if (first) v0 = val[0];  // first valid cut: the shift
+            first = false;
 #pragma unroll
             for (int g = 0; g < G; ++g) {
-#pragma unroll
-                for (int q = 0; q < NCH; ++q) {
-                    const float d = __fmul_rn(__fsub_rn(val[g][q], v0[q]), keep[g]);
-                    s1[q] = __fadd_rn(s1[q], d);
-                    s2[q] = __fmaf_rn(d, d, s2[q]);
-                }
+                if (g >= have) break;
+                const float d = __fsub_rn(val[g], v0);
+                s1 = __fadd_rn(s1, d);
+                s2 = __fmaf_rn(d, d, s2);
             }
         }
     }
+    return lane_sum(n >= 2 ? kTermScale * double(__fsub_rn(__fmul_rn(float(n), s2), __fmul_rn(s1, s1))) : 0.0);
+}
+
+// The last, partial chunk (tail < 32 samples) of several trials at once: groups
+// of `width` lanes (a power of two >= tail), each its own trial t with its own
+// valid cuts; every lane of the warp calls it.  The same sums as
+// trial_chunk's with the lanes past the tail contributing zero.
+template <bool STAGED>
+__device__ __forceinline__ double trial_tail(const TrialLines& lines, const SampleArea<STAGED>& A, int t,
+                                             uint32_t valid, int k, bool live, int width)
+{
+    constexpr int G = 4;
+    const int n = __popc(valid);
+    float v0 = 0.f, s1 = 0.f, s2 = 0.f;
+    const float kf = float(k);
+    bool first = true;
+    for (uint32_t m = n >= 2 ? valid : 0u; __any_sync(0xffffffffu, m != 0u);) {
+        float val[G];
+        bool use[G];
 #pragma unroll
-    for (int q = 0; q < NCH; ++q) {
-        const double term =
-            (n >= 2 && act[q]) ? double(__fsub_rn(__fmul_rn(float(n), s2[q]), __fmul_rn(s1[q], s1[q]))) : 0.0;
-        out[q] = lane_sum(term);
+        for (int g = 0; g < G; ++g) {
+            use[g] = m != 0u;
+            const int c = m ? __ffs(m) - 1 : 0;
+            m &= m - 1;
+            const int i = t * lines.stride + c;
+            val[g] = use[g] ? cut_sample(A, lines.uv[i], lines.w[i], kf) : 0.f;
+        }
+        if (first) v0 = val[0];
+        first = false;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const float d = use[g] ? __fsub_rn(val[g], v0) : 0.f;
+            s1 = __fadd_rn(s1, d);
+            s2 = __fmaf_rn(d, d, s2);
+        }
     }
+    double v = (n >= 2 && live) ? kTermScale * double(__fsub_rn(__fmul_rn(float(n), s2), __fmul_rn(s1, s1))) : 0.0;
+    for (int o = width >> 1; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// The sampling tasks of a round, spread over the warps of the cluster: one per
+// trial and whole chunk, chunk by chunk (a block keeps to a band of the
+// marker), then the packed partial chunks; `valid` is trial `lane`'s cuts.
+struct Tasks {
+    int nTrials, whole, tail, width, packed;  // whole chunks, samples of the last one, its lanes, its trials per warp
+    __device__ int nWhole() const { return nTrials * whole; }
+    __device__ int count() const { return nWhole() + (tail ? (nTrials + packed - 1) / packed : 0); }
+};
+template <bool STAGED>
+__device__ __forceinline__ void sample_round(Shared& S, const TrialLines& lines, const SampleArea<STAGED>& A,
+                                             const Tasks& K, uint32_t valid, int par, int first, int step, int csize,
+                                             int lane)
+{
+    // every block of the cluster gets every share: lane q stores to block q
+    namespace cg = cooperative_groups;
+    auto put = [&](int j, int t, double c, int from, int by) {
+        if (csize == 1) {
+            if (from == 0) S.part[par][j][t] = c;
+        } else {
+            for (int q = from; q < csize; q += by) *cg::this_cluster().map_shared_rank(&S.part[par][j][t], q) = c;
+        }
+    };
+    for (int task = first; task < K.count(); task += step) {
+        if (task < K.nWhole()) {
+            const int j = task / K.nTrials, t = task - j * K.nTrials;
+            const double c = trial_chunk(lines, A, t, __shfl_sync(0xffffffffu, valid, t), j * kChunk + lane);
+            put(j, t, c, lane, 32);
+        } else {
+            const int own = (task - K.nWhole()) * K.packed + lane / K.width, t = min(own, K.nTrials - 1);
+            const int k = lane % K.width;
+            const bool live = k < K.tail && own < K.nTrials;  // each lane of the group ends with its sum
+            const double c = trial_tail(lines, A, t, __shfl_sync(0xffffffffu, valid, t),
+                                        K.whole * kChunk + min(k, K.tail - 1), live, K.width);
+            if (own < K.nTrials) put(K.whole, t, c, k, K.width);
+        }
+    }
+}
+
+// Ascending sort of a thread's 32 values: Batcher's odd-even merge network
+// (K. E. Batcher, "Sorting networks and their applications", AFIPS 1968), its
+// steps as templates so that every index is a constant (registers only).
+template <int P, int K>
+__device__ __forceinline__ void sort_network(float (&v)[kMaxCuts])
+{
+    static_assert(kMaxCuts == 32, "a power of two");
+#pragma unroll
+    for (int j = K % P; j + K < kMaxCuts; j += 2 * K)
+#pragma unroll
+        for (int i = j; i < j + K; ++i)
+            if (i + K < kMaxCuts && i / (2 * P) == (i + K) / (2 * P)) {
+                const float a = v[i], b = v[i + K];
+                v[i] = fminf(a, b);
+                v[i + K] = fmaxf(a, b);
+            }
+    if constexpr (K > 1) sort_network<P, K / 2>(v);
+    else if constexpr (2 * P < kMaxCuts) sort_network<2 * P, 2 * P>(v);
 }
 
 // Identification.hpp:373-384, with val = +1 (white: even ratio count) or -1
@@ -521,8 +774,9 @@ __device__ __forceinline__ void inverse_derivative(const float* Hi, const float*
 // Sample k of a cut for Gauss-Newton at the trial homography S.gH: its value
 // and, in ds, its derivatives along the two center coordinates (through H, and
 // through the back-projected cut end (bx, by) whose derivatives are db).
-__device__ __forceinline__ float gn_sample(const Shared& S, const Roi& roi, float bs, float den, float bx, float by,
-                                          const float db[2][2], int k, float ds[2])
+template <bool STAGED>
+__device__ __forceinline__ float gn_sample(const Shared& S, const SampleArea<STAGED>& area, float bs, float den,
+                                          float bx, float by, const float db[2][2], int k, float ds[2])
 {
     const float xs = bx * bs, ys = by * bs;
     const float sx = (bx - xs) / den, sy = (by - ys) / den;
@@ -534,7 +788,12 @@ __device__ __forceinline__ float gn_sample(const Shared& S, const Roi& roi, floa
     const float r = __frcp_rn(w);
     const float qx = __fmul_rn(u, r), qy = __fmul_rn(v, r);
     float gx, gy;
-    const float val = bilinear_grad(roi, qx, qy, gx, gy);
+    uint32_t pb[4];
+    float p[4], fx, fy;
+    area_taps(area, qx, qy, pb, fx, fy);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) p[q] = byte_to_float(pb[q]);
+    const float val = bilinear_value_grad(p, fx, fy, gx, gy);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         const float* dH = S.gdH[q];
@@ -599,24 +858,23 @@ __device__ __forceinline__ void gn_chunk_sums(uint32_t valid, int n, bool live, 
 // sum of squares is the reference's pair cost up to the factor n / pairs;
 // Jacobian d r_ik / d center from the forward derivatives of the trial
 // homography, its inverse (which moves the back-projected cut ends) and the
-// bilinear patch.  Each block of the cluster sums its samples; the sums meet
+// bilinear patch.  Each block of the cluster sums its chunks; the sums meet
 // through distributed shared memory and every block takes the same step.
 // Starts from the grid's center; a step that raises the cost is rejected and
 // the damping raised.  Stops when a step is below 1e-3 px, or after
 // gnIterations cost evaluations.
-template <int CL>
-__device__ void gn_refine(Shared& S, const IdentTask& T, const Roi& roi, const IdentParams& ip, uint32_t cutMask,
-                          int crank)
+template <bool CLUSTER>
+__device__ void gn_refine(Shared& S, void* work, const uint8_t* px, const IdentTask& T, const Roi& roi,
+                          const IdentParams& ip, uint32_t cutMask, int crank, int csize)
 {
     namespace cg = cooperative_groups;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nthreads = blockDim.x, nwarps = nthreads >> 5;
+    GnChunk& chunk = *static_cast<GnChunk*>(work);
     const int nS = ip.nSamples;
     const int nch = (nS + kChunk - 1) / kChunk;
     const float bs = ip.beginSig;
     const float den = float(nS) - 1.f;
-    // chunks of this block: all of them, or chunk `crank` in a cluster
-    const int j0 = CL == 1 ? 0 : crank;
-    const int j1 = CL == 1 ? nch : min(crank + 1, nch);
     if (tid == 0) {
         S.gTry[0] = S.cx;
         S.gTry[1] = S.cy;
@@ -637,9 +895,21 @@ __device__ void gn_refine(Shared& S, const IdentTask& T, const Roi& roi, const I
         }
         __syncthreads();
         if (S.gStop) break;
-        // cuts whose end samples leave the rectangle at this center
+        // cuts whose end samples leave the rectangle at this center, and (once
+        // per cut) their back-projected ends
+        if (warp == nwarps - 1 && lane < T.ncuts) {
+            float bx, by, db[2][2];
+            back_project(S.gHi, S.gdHi[0], S.gdHi[1], T.stop[lane][0], T.stop[lane][1], bx, by, db);
+            float* o = S.gBack[lane];
+            o[0] = bx;
+            o[1] = by;
+            o[2] = db[0][0];
+            o[3] = db[0][1];
+            o[4] = db[1][0];
+            o[5] = db[1][1];
+        }
         if (warp == 0) {
-            bool bad = false;
+            bool bad = false, out = false;
             if (lane < T.ncuts) {
                 float bx, by, w;
                 apply_h(S.gHi, T.stop[lane][0], T.stop[lane][1], bx, by, w);
@@ -650,68 +920,91 @@ __device__ void gn_refine(Shared& S, const IdentTask& T, const Roi& roi, const I
                 apply_h(S.gH, xs + den * sx, ys + den * sy, x1, y1, w1);
                 bad = !(w0 > 0.f && w1 > 0.f) && !(w0 < 0.f && w1 < 0.f);
                 bad = bad || !inside(roi, x0, y0) || !inside(roi, x1, y1);
+                out = !bad && !(in_box(S, roi, x0, y0) && in_box(S, roi, x1, y1));
             }
             const uint32_t m = __ballot_sync(0xffffffffu, bad);
-            if (lane == 0) S.gOob = m & cutMask;
+            out = __any_sync(0xffffffffu, out);
+            if (lane == 0) {
+                S.gOob = m & cutMask;
+                S.direct = out;
+            }
         }
         __syncthreads();
         const uint32_t valid = ~(S.oob | S.gOob) & cutMask;
         const int n = __popc(valid);
         const int par = it & 1;
-        // One block doing every chunk, with room for all samples: each warp
-        // computes its cuts' samples of every chunk (the back-projected end
-        // once per cut), then warp j sums chunk j.  The per-chunk sums are
-        // the same operations in the same order as the chunk-at-a-time path,
-        // so both give the same bits.
-        const bool whole = CL == 1 && 2 * T.ncuts * nS <= int(sizeof(S.u) / sizeof(float));
-        if (whole) {
-            float* gdx = reinterpret_cast<float*>(&S.u);
-            float* gdy = gdx + T.ncuts * nS;
-            for (int c = warp; c < T.ncuts; c += kWarps) {
-                if (!((valid >> c) & 1u)) continue;
-                float bx, by, db[2][2];
-                back_project(S.gHi, S.gdHi[0], S.gdHi[1], T.stop[c][0], T.stop[c][1], bx, by, db);
-                for (int k = lane; k < nS; k += kChunk) {
-                    float ds[2];
-                    S.sig[c][k] = gn_sample(S, roi, bs, den, bx, by, db, k, ds);
-                    gdx[c * nS + k] = ds[0];
-                    gdy[c * nS + k] = ds[1];
-                }
-            }
-            __syncthreads();
-            if (warp < nch) {
-                const int k = warp * kChunk + lane;
+        // One block doing every chunk, with room for all samples: the threads
+        // compute the samples, then a warp sums a chunk.  The per-chunk sums
+        // are the same operations in the same order as the chunk-at-a-time
+        // path, so both give the same bits.
+        const bool direct = S.direct;
+        auto sample = [&](int c, int k, float ds[2]) {
+            const float* o = S.gBack[c];
+            const float db[2][2] = {{o[2], o[3]}, {o[4], o[5]}};
+            return direct ? gn_sample(S, image_area(roi), bs, den, o[0], o[1], db, k, ds)
+                          : gn_sample(S, staged_area(S, px), bs, den, o[0], o[1], db, k, ds);
+        };
+        if (!CLUSTER && nwarps <= kMaxChunks) {
+            // a small block, one of several on its SM: a warp takes a chunk's
+            // samples and sums them as they come
+            for (int j = warp; j < nch; j += nwarps) {
+                const int k = j * kChunk + lane;
                 double acc[6];
                 gn_chunk_sums(valid, n, k < nS, acc, [&](int c, float& v, float& a, float& b) {
-                    v = S.sig[c][k];
+                    float ds[2];
+                    v = sample(c, k, ds);
+                    a = ds[0];
+                    b = ds[1];
+                });
+                if (lane == 0)
+#pragma unroll
+                    for (int q = 0; q < 6; ++q) S.gPart[par][j][q] = acc[q];
+            }
+            __syncthreads();
+        } else if (!CLUSTER && T.ncuts * nS <= kGnWhole) {
+            float* gs = static_cast<float*>(work);
+            float* gdx = gs + kGnWhole;
+            float* gdy = gdx + kGnWhole;
+            for (int i = tid; i < T.ncuts * nS; i += nthreads) {
+                const int c = i / nS;
+                if (!((valid >> c) & 1u)) continue;
+                float ds[2];
+                gs[i] = sample(c, i - c * nS, ds);
+                gdx[i] = ds[0];
+                gdy[i] = ds[1];
+            }
+            __syncthreads();
+            for (int j = warp; j < nch; j += nwarps) {
+                const int k = j * kChunk + lane;
+                double acc[6];
+                gn_chunk_sums(valid, n, k < nS, acc, [&](int c, float& v, float& a, float& b) {
+                    v = gs[c * nS + k];
                     a = gdx[c * nS + k];
                     b = gdy[c * nS + k];
                 });
                 if (lane == 0)
 #pragma unroll
-                    for (int q = 0; q < 6; ++q) S.gPart[par][warp][q] = acc[q];
+                    for (int q = 0; q < 6; ++q) S.gPart[par][j][q] = acc[q];
             }
             __syncthreads();
         } else {
-            for (int j = j0; j < j1; ++j) {
+            for (int j = crank; j < nch; j += csize) {
                 // this chunk's samples: value and its derivatives along the center
                 const int k = j * kChunk + lane;
-                for (int c = warp; c < T.ncuts; c += kWarps) {
+                for (int c = warp; c < T.ncuts; c += nwarps) {
                     if (!((valid >> c) & 1u) || k >= nS) continue;
-                    float bx, by, db[2][2];
-                    back_project(S.gHi, S.gdHi[0], S.gdHi[1], T.stop[c][0], T.stop[c][1], bx, by, db);
                     float ds[2];
-                    S.u.gn.s[c][lane] = gn_sample(S, roi, bs, den, bx, by, db, k, ds);
-                    S.u.gn.dx[c][lane] = ds[0];
-                    S.u.gn.dy[c][lane] = ds[1];
+                    chunk.s[c][lane] = sample(c, k, ds);
+                    chunk.dx[c][lane] = ds[0];
+                    chunk.dy[c][lane] = ds[1];
                 }
                 __syncthreads();
                 if (warp == 0) {
                     double acc[6];
                     gn_chunk_sums(valid, n, k < nS, acc, [&](int c, float& v, float& a, float& b) {
-                        v = S.u.gn.s[c][lane];
-                        a = S.u.gn.dx[c][lane];
-                        b = S.u.gn.dy[c][lane];
+                        v = chunk.s[c][lane];
+                        a = chunk.dx[c][lane];
+                        b = chunk.dy[c][lane];
                     });
                     if (lane == 0)
 #pragma unroll
@@ -722,12 +1015,12 @@ __device__ void gn_refine(Shared& S, const IdentTask& T, const Roi& roi, const I
         }
         // every chunk's sums are in; a parity's array is rewritten two
         // evaluations later, past the next barrier of the cluster
-        if constexpr (CL > 1) cg::this_cluster().sync();
+        if constexpr (CLUSTER) cg::this_cluster().sync();
         if (warp == 0 && lane < 6) {
             double a = 0.0;
             for (int j = 0; j < nch; ++j) {
                 const double* src = &S.gPart[par][j][0];
-                if constexpr (CL > 1) src = cg::this_cluster().map_shared_rank(src, j);
+                if constexpr (CLUSTER) src = cg::this_cluster().map_shared_rank(src, j % csize);
                 a += src[lane];
             }
             S.gSum[lane] = a;
@@ -776,35 +1069,31 @@ __device__ void gn_refine(Shared& S, const IdentTask& T, const Roi& roi, const I
 
 }  // namespace
 
-// CL = 1: one block per marker; CL = kCluster: a cluster of blocks per marker
-// (launched with that cluster dimension), block r on sample chunk r.  MB:
-// blocks per SM the registers are budgeted for (2 suits Gauss-Newton, whose
-// steps leave most warps waiting; the grid keeps every warp busy and prefers
-// the registers).  The register caps follow from the 25 warps of a block
-// spread over the SM's four 16 K-register partitions (7 warps on one): 72 for
-// one block per SM, 32 for two; 64 for the cluster form (the detection's),
-// which needs no spill at 64 and so leaves room in every partition for a
-// block of another stream's kernel.
-template <int CL, int MB>
-__global__ void __maxnreg__(CL > 1 ? 64 : (MB == 1 ? 72 : 32))
+// One marker per cluster (CLUSTER, blocks of one marker side by side) or per
+// block; any number of warps.  72 registers: 25 warps on an SM put 7 on one of
+// its four register partitions (five blocks of 5 warps, or one of 20).
+template <bool CLUSTER>
+__global__ void __maxnreg__(72)
     k_identify(const uint8_t* __restrict__ img, size_t pitch, const IdentTask* __restrict__ tasks, IdentResult* res,
-               const float* __restrict__ bankInv, IdentParams ip)
+               const float* __restrict__ bankInv, IdentParams ip, int workBytes, int boxBytes)
 {
     namespace cg = cooperative_groups;
     __shared__ Shared S;
-    int crank = 0;
-    if constexpr (CL > 1) crank = int(cg::this_cluster().block_rank());
-    const int marker = blockIdx.x / CL;
+    extern __shared__ float4 work[];  // workBytes, then room for boxBytes of pixels; at least FinalWork
+    uint8_t* const px = reinterpret_cast<uint8_t*>(work) + workBytes;
+    FinalWork& F = *reinterpret_cast<FinalWork*>(work);
+    int crank = 0, csize = 1;
+    if constexpr (CLUSTER) {
+        crank = int(cg::this_cluster().block_rank());
+        csize = int(cg::this_cluster().num_blocks());
+    }
+    const int marker = blockIdx.x / csize;
     const IdentTask& T = tasks[marker];
     const Roi roi = make_roi(img, pitch, T);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nthreads = blockDim.x, nwarps = nthreads >> 5;
     const int nS = ip.nSamples;
     const int nch = (nS + kChunk - 1) / kChunk;
-    // chunks this block evaluates (all, or chunk `crank` in a cluster), NCH
-    // per pass (fewer live registers when two blocks share an SM)
-    constexpr int NCH = CL == 1 ? (MB == 1 ? kMaxChunks : kMaxChunks / 2) : 1;
-    const int j0 = CL == 1 ? 0 : crank;
-    const int jEnd = CL == 1 ? nch : j0 + 1;
     const int gridN = ip.gridN;
     const int nTrials = gridN * gridN;
     const uint32_t cutMask = (T.ncuts >= 32) ? 0xffffffffu : ((1u << T.ncuts) - 1u);
@@ -858,64 +1147,80 @@ __global__ void __maxnreg__(CL > 1 ? 64 : (MB == 1 ? 72 : 32))
         S.rounds = r;
         S.iterations = r;
     }
+    if (warp == 2) find_box(S, T, roi, size_t(boxBytes), lane);
+    if (tid == 32) {  // plane radii of the samples, by the reference's running sum
+        const float step = (1.f - ip.beginSig) / (float(nS) - 1.f);
+        float x = ip.beginSig;
+        for (int k = 0; k < nS; ++k) {
+            S.radius[k] = x;
+            x += step;
+        }
+    }
+    for (int i = tid; i <= kMaxSamples; i += nthreads) S.rcp[i] = __frcp_rn(float(i));
     __syncthreads();
+    stage_box(S, roi, px);
+    asm volatile("cp.async.wait_all;" ::: "memory");  // before the first barrier below
+    const TrialLines lines = trial_lines(work, nTrials, T.ncuts);
+    Tasks K{nTrials, nS / kChunk, nS % kChunk, 1, 0};
+    while (K.width < K.tail) K.width <<= 1;
+    K.packed = kChunk / K.width;
     float ns = ip.neighbourSize;
     for (int round = 0; round < S.rounds; ++round) {
-        // getNearbyPoints (Identification.cpp:1071-1109)
-        if (warp < nTrials) {
+        // getNearbyPoints (Identification.cpp:1071-1109): a lane per trial
+        if (tid == 32) S.direct = 0;
+        if (warp == 0 && lane < nTrials) {
             const float size = ns * S.nsScale;
             const float half = size / 2.f, step = size / float(gridN - 1);
             const float ccx = S.mT[0] * S.cx + S.mT[1] * S.cy + S.mT[2];
             const float ccy = S.mT[3] * S.cx + S.mT[4] * S.cy + S.mT[5];
-            const int i = warp / gridN, j = warp % gridN;
+            const int i = lane / gridN, j = lane % gridN;
             const float qx = ccx - half + float(i) * step, qy = ccy - half + float(j) * step;
             float px, py, w;
             apply_h(S.mTi, qx, qy, px, py, w);
-            setup_trial(S, T, warp, px, py, ip, roi, lane);
-        }
-        __syncthreads();
-        // sticky out-of-bounds flags in trial order: inclusive OR scan
-        if (warp == 0) {
-            uint32_t m = lane < nTrials ? S.trialOob[lane] : 0u;
+            float Hm[9], Hi[9];
+            homography_from_center(S.C, S.Tp, S.Td, px, py, Hm);
+            const bool ok = mat_inv(Hm, Hi);
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, m, o);
-                if (lane >= o) m |= v;
+            for (int k = 0; k < 9; ++k) {
+                S.trialH[lane][k] = Hm[k];
+                S.trialHi[lane][k] = Hi[k];
             }
-            m |= S.oob;
-            if (lane < nTrials) S.valid[lane] = ~m & cutMask;
-            const uint32_t last = __shfl_sync(0xffffffffu, m, nTrials - 1);
-            __syncwarp();
-            if (lane == 0) S.oob = last;
+            S.trialOk[lane] = ok;
+            S.trialOob[lane] = 0u;
+            S.trialPt[lane][0] = px;
+            S.trialPt[lane][1] = py;
         }
         __syncthreads();
+        for (int i = tid; i < nTrials * T.ncuts; i += nthreads) {
+            const int t = i / T.ncuts;
+            setup_cut(S, lines, T, t, i - t * T.ncuts, ip, roi);
+        }
+        __syncthreads();
+        // sticky out-of-bounds flags in trial order (every warp for itself):
+        // inclusive OR scan; lane t then holds trial t's valid cuts
+        uint32_t flags = lane < nTrials ? S.trialOob[lane] : 0u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, flags, o);
+            if (lane >= o) flags |= v;
+        }
+        flags |= S.oob;
+        const uint32_t valid = lane < nTrials ? ~flags & cutMask : 0u;
         const int par = round & 1;
-        if (warp < nTrials) {
-            for (int jp = j0; jp < jEnd; jp += NCH) {
-                double c[NCH];
-                trial_partial<NCH>(S, roi, warp, S.valid[warp], jp, nch, nS, lane, c);
-                if (lane == 0)
-#pragma unroll
-                    for (int q = 0; q < NCH; ++q)
-                        if (jp + q < nch) S.part[par][jp + q][warp] = c[q];
-            }
-        }
-        // All chunks of the marker are in; a block rewrites this parity's
-        // array two rounds later, after the next cluster barrier, when every
-        // block has finished reading it.
-        if constexpr (CL > 1) cg::this_cluster().sync();
+        const int firstTask = crank * nwarps + warp, stepTask = csize * nwarps;
+        if (S.direct) sample_round(S, lines, image_area(roi), K, valid, par, firstTask, stepTask, csize, lane);
+        else sample_round(S, lines, staged_area(S, px), K, valid, par, firstTask, stepTask, csize, lane);
+        // All chunks of the marker are in, in every block; this parity's array
+        // is written again two rounds later, after the next cluster barrier,
+        // when every block has finished reading it.
+        if constexpr (CLUSTER) cg::this_cluster().sync();
         else __syncthreads();
         if (warp == 0) {
             double acc = 0.0;
             if (lane < nTrials)
-                for (int j = 0; j < nch; ++j) {
-                    const double* src = &S.part[par][j][0];
-                    if constexpr (CL > 1) src = cg::this_cluster().map_shared_rank(src, j);
-                    acc += src[lane];
-                }
-            const int n = lane < nTrials ? __popc(S.valid[lane]) : 0;
+                for (int j = 0; j < nch; ++j) acc += S.part[par][j][lane];
+            const int n = __popc(valid);
             const float cost = n >= 2 ? float(acc / (0.5 * double(n) * double(n - 1))) : FLT_MAX;
-            if (lane < nTrials) S.cost[lane] = cost;
             // imageCenterOptimizationGlob: first strict minimum in trial order
             // (costs below FLT_MAX; key = orderable cost bits, then index)
             unsigned long long key = ~0ull;
@@ -930,17 +1235,18 @@ __global__ void __maxnreg__(CL > 1 ? 64 : (MB == 1 ? 72 : 32))
                 key = k2 < key ? k2 : key;
             }
             const bool readable = __any_sync(0xffffffffu, n >= 2);
-            __syncwarp();
+            const uint32_t last = __shfl_sync(0xffffffffu, flags, nTrials - 1);
+            const int bi = int(key & 0xffffffffull);
+            const bool found = readable && key != ~0ull;
+            if (found && lane < 9) S.Hopt[lane] = S.trialH[bi][lane];
+            if (found && lane == bi) {
+                S.cx = S.trialPt[bi][0];
+                S.cy = S.trialPt[bi][1];
+                S.minRes = cost;
+            }
             if (lane == 0) {
-                if (!readable || key == ~0ull) {
-                    S.fail = 1;
-                } else {
-                    const int bi = int(key & 0xffffffffull);
-                    S.cx = S.trialPt[bi][0];
-                    S.cy = S.trialPt[bi][1];
-                    for (int k = 0; k < 9; ++k) S.Hopt[k] = S.trialH[bi][k];
-                    S.minRes = S.cost[bi];
-                }
+                S.oob = last;
+                if (!found) S.fail = 1;
             }
         }
         __syncthreads();
@@ -948,196 +1254,237 @@ __global__ void __maxnreg__(CL > 1 ? 64 : (MB == 1 ? 72 : 32))
         ns /= float((gridN - 1) / 2);
     }
     if (ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON && !S.fail && S.rounds > 0)
-        gn_refine<CL>(S, T, roi, ip, cutMask, crank);
-    // No block leaves while another may still read its shared memory; the
-    // rest of the identification runs in the first block of the cluster.
-    if constexpr (CL > 1) {
-        cg::this_cluster().sync();
-        if (crank != 0) return;
-    }
+        gn_refine<CLUSTER>(S, work, px, T, roi, ip, cutMask, crank, csize);
+    const bool read = !S.fail && S.rounds > 0;
     IdentResult& R = res[marker];
-    if (S.fail || S.rounds == 0) {
-        if (tid == 0) {
-            R.status = CCTAGB_OPTI_HAS_DIVERGED;
-            R.id = -1;
-            R.x = S.cx;
-            R.y = S.cy;
-            for (int k = 0; k < 9; ++k) R.H[k] = 0.f;
-            R.residual = FLT_MAX;
-            R.score = 0.f;
-            R.nvalid = 0;
-            R.iterations = S.iterations;
-        }
+    if (!read && tid == 0 && crank == 0) {
+        R.status = CCTAGB_OPTI_HAS_DIVERGED;
+        R.id = -1;
+        R.x = S.cx;
+        R.y = S.cy;
+        for (int k = 0; k < 9; ++k) R.H[k] = 0.f;
+        R.residual = FLT_MAX;
+        R.score = 0.f;
+        R.nvalid = 0;
+        R.iterations = S.iterations;
+    }
+    // The reading of the cuts is spread over the cluster: the first block takes
+    // the signals of all cuts, for the barcode; the others (or the only one) the
+    // cuts' distances to the bank, a share each.  No block leaves while another
+    // may still use its shared memory.
+    if (!read) {
+        if constexpr (CLUSTER) cg::this_cluster().sync();
         return;
     }
+    const int shares = csize > 1 ? csize - 1 : 1, share = csize > 1 ? crank - 1 : 0;  // share -1: none
+    auto mine = [&](int c) { return share >= 0 && c % shares == share; };
     // Final signals with the optimal homography (getSignals, Identification.cpp:901).
-    for (int c = warp; c < T.ncuts; c += kWarps) {
+    {
         float Hi[9];
         mat_inv(S.Hopt, Hi);
-        float bx, by, w;
-        apply_h(Hi, T.stop[c][0], T.stop[c][1], bx, by, w);
-        const float xs = bx * ip.beginSig, ys = by * ip.beginSig;
-        const float sx = (bx - xs) / (float(nS) - 1.f), sy = (by - ys) / (float(nS) - 1.f);
-        bool bad = false;
-        for (int k = lane; k < nS; k += 32) {
-            const float x = xs + float(k) * sx, y = ys + float(k) * sy;
-            float xr, yr;
-            apply_h(S.Hopt, x, y, xr, yr, w);
-            if (inside(roi, xr, yr)) S.sig[c][k] = bilinear(roi, xr, yr);
-            else bad = true;
+        __syncthreads();  // the rounds' use of the work area is over
+        const int first = crank == 0 ? 0 : share, step = crank == 0 ? 1 : shares;
+        for (int c = first + step * warp; c < T.ncuts; c += step * nwarps) {
+            float bx, by, w;
+            apply_h(Hi, T.stop[c][0], T.stop[c][1], bx, by, w);
+            const float xs = bx * ip.beginSig, ys = by * ip.beginSig;
+            const float sx = (bx - xs) / (float(nS) - 1.f), sy = (by - ys) / (float(nS) - 1.f);
+            bool bad = false;
+#pragma unroll
+            for (int q = 0; q < kMaxChunks; ++q) {
+                const int k = q * 32 + lane;
+                if (k >= nS) continue;
+                const float x = xs + float(k) * sx, y = ys + float(k) * sy;
+                float xr, yr;
+                apply_h(S.Hopt, x, y, xr, yr, w);
+                if (inside(roi, xr, yr)) F.sig[c][k] = bilinear(roi, xr, yr);
+                else bad = true;
+            }
+            const uint32_t any = __ballot_sync(0xffffffffu, bad);
+            if (lane == 0 && any) atomicOr(&S.oob, 1u << c);
         }
-        const uint32_t any = __ballot_sync(0xffffffffu, bad);
-        if (lane == 0 && any) atomicOr(&S.oob, 1u << c);
+    }
+    // Bank row i sees a sample as black when it lies inside an odd number of its
+    // rings (1 / ratio <= radius): per ring, all samples from the first one at
+    // least that far out flip.
+    for (int i = tid; share >= 0 && i < ip.nIds; i += nthreads) {
+        uint32_t bits[kMaxSamples / 32] = {};
+        for (int r = 0; r < ip.nRatios; ++r) {
+            const float inv = __ldg(&bankInv[i * kMaxBankRatios + r]);
+            int k = min(max(int((inv - ip.beginSig) / (1.f - ip.beginSig) * (float(nS) - 1.f)), 0), nS);
+            while (k > 0 && S.radius[k - 1] >= inv) --k;
+            while (k < nS && S.radius[k] < inv) ++k;
+#pragma unroll
+            for (int w = 0; w < kMaxSamples / 32; ++w)
+                bits[w] ^= k <= 32 * w ? 0xffffffffu : k >= 32 * w + 32 ? 0u : 0xffffffffu << (k - 32 * w);
+        }
+#pragma unroll
+        for (int w = 0; w < kMaxSamples / 32; ++w) F.black[i][w] = bits[w];
     }
     __syncthreads();
-    const uint32_t valid = ~S.oob & cutMask;
+    const uint32_t valid = ~S.oob & cutMask;  // beyond the first block: of its own cuts
     const int nValid = __popc(valid);
-    // Median barcode over the valid cuts (computeMedian, Identification.hpp:351-371).
-    if (tid < nS) {
-        float v[kMaxCuts];
-        int n = 0;
-        uint32_t m = valid;
-        while (m) {
-            const int c = __ffs(m) - 1;
-            m &= m - 1;
-            const float x = S.sig[c][tid];
-            int j = n++;
-            while (j > 0 && v[j - 1] > x) {
-                v[j] = v[j - 1];
-                --j;
-            }
-            v[j] = x;
-        }
-        float med = 0.f;
-        if (n > 0) med = (n & 1) ? v[n / 2] : float((double(v[n / 2]) + double(v[n / 2 - 1])) / 2.0);
-        S.barcode[tid] = med;
-    }
-    __syncthreads();
-    // Orazio distance per valid cut: lane = bank id (Identification.cpp:77-190).
-    for (int c = warp; c < T.ncuts; c += kWarps) {
-        if (!((valid >> c) & 1u)) continue;
-        const float* sg = S.sig[c];
-        // statistics over samples [30, n): Boost immediate mean / variance
-        // (the divisions by the counts correctly rounded by div_small)
-        float mean = 0.f, var = 0.f;
-        {
-            int cnt = 0;
-            float rprev = 1.f;
+    // Statistics of each cut's signal (Identification.cpp:77-190), a lane per cut
+    // (the last warp: the first ones sort meanwhile).
+    if (warp == nwarps - 1) {
+        const int c = lane;
+        if (c < T.ncuts && mine(c) && ((valid >> c) & 1u)) {
+            const float* sg = F.sig[c];
+            // over samples [30, n): Boost immediate mean / variance (the
+            // divisions by the counts correctly rounded by div_small)
+            float mean = 0.f, var = 0.f;
+#pragma unroll 4
             for (int k = 30; k < nS; ++k) {
-                ++cnt;
+                const int cnt = k - 29;
                 const float x = sg[k];
-                const float fc = float(cnt), fc1 = float(cnt - 1), rc = __frcp_rn(fc);
+                const float fc = float(cnt), fc1 = float(cnt - 1), rc = S.rcp[cnt];
                 mean = pm::div_small(__fmaf_rn(mean, fc1, x), fc, rc);
-                if (cnt > 1) {
-                    const float t = __fsub_rn(x, mean);
-                    var = __fadd_rn(pm::div_small(__fmul_rn(var, fc1), fc, rc),
-                                    pm::div_small(__fmul_rn(t, t), fc1, rprev));
-                }
-                rprev = rc;
+                const float t = __fsub_rn(x, mean);
+                const float v = __fadd_rn(pm::div_small(__fmul_rn(var, fc1), fc, rc),
+                                          pm::div_small(__fmul_rn(t, t), fc1, S.rcp[cnt - 1]));
+                if (cnt > 1) var = v;
             }
-        }
-        float mub = 0.f, muw = 0.f;
-        {
-            int ni = 0, nsup = 0;
-            bool acc = false;
+            // running means of the samples below the mean and of the others,
+            // from the first one below it
+            float mub = 0.f, muw = 0.f;
+            int nb = 0, nw = 0;
+#pragma unroll 4
             for (int k = 0; k < nS; ++k) {
                 const float x = sg[k];
-                if (!acc && x < mean) acc = true;
-                if (acc) {
-                    if (x < mean) {
-                        ++ni;
-                        mub = pm::div_small(__fmaf_rn(mub, float(ni - 1), x), float(ni), __frcp_rn(float(ni)));
-                    } else {
-                        ++nsup;
-                        muw = pm::div_small(__fmaf_rn(muw, float(nsup - 1), x), float(nsup),
-                                            __frcp_rn(float(nsup)));
-                    }
-                }
+                const bool below = x < mean, use = below || nb > 0;
+                const int n1 = below ? nb : nw;
+                const float mu = below ? mub : muw;
+                const float m = pm::div_small(__fmaf_rn(mu, float(n1), x), float(n1 + 1), S.rcp[n1 + 1]);
+                mub = use && below ? m : mub;
+                muw = use && !below ? m : muw;
+                nb += below ? 1 : 0;
+                nw += use && !below ? 1 : 0;
+            }
+            // dis()'s division by 2 var: a float quotient through the double
+            // reciprocal is correctly rounded for a normal result (its relative
+            // error, 2^-52, is below the 2^-49 that separates a quotient of floats
+            // from a float rounding midpoint), so each term is the IEEE quotient.
+            const double rvar2 = 1.0 / double(2.0f * var);
+            S.stats[c][0] = mub;
+            S.stats[c][1] = muw;
+            S.stats[c][2] = __int_as_float(__double2hiint(rvar2));
+            S.stats[c][3] = __int_as_float(__double2loint(rvar2));
+        }
+    }
+    // Median barcode over the valid cuts (computeMedian, Identification.hpp:
+    // 351-371): a thread per sample sorts its values in registers by Batcher's
+    // odd-even merge network, absent cuts last.
+    if (crank == 0)
+        for (int k = tid; k < nS; k += nthreads) {
+            float v[kMaxCuts];
+#pragma unroll
+            for (int c = 0; c < kMaxCuts; ++c) v[c] = c < T.ncuts && ((valid >> c) & 1u) ? F.sig[c][k] : FLT_MAX;
+            sort_network<1, 1>(v);
+            float hi = 0.f, lo = 0.f;
+#pragma unroll
+            for (int c = 0; c < kMaxCuts; ++c) {
+                hi = c == nValid / 2 ? v[c] : hi;
+                lo = c == nValid / 2 - 1 ? v[c] : lo;
+            }
+            F.barcode[k] = nValid == 0 ? 0.f : (nValid & 1) ? hi : float((double(hi) + double(lo)) / 2.0);
+        }
+    __syncthreads();
+    // Orazio distance per valid cut, a warp per cut, lane = bank id (four rows of
+    // 32): a sample adds one of two terms, by the row's black mask, in order.
+    // The terms sit in the lanes' registers, sample k's in lane k mod 32.
+    for (int c = share + shares * warp; share >= 0 && c < T.ncuts; c += shares * nwarps) {
+        if (!((valid >> c) & 1u)) continue;
+        const float mub = S.stats[c][0], muw = S.stats[c][1];
+        const double rvar2 = __hiloint2double(__float_as_int(S.stats[c][2]), __float_as_int(S.stats[c][3]));
+        float dist[kMaxBankIds / 32] = {};
+        for (int w = 0; w < nch; ++w) {
+            const int k = 32 * w + lane;
+            // past the last sample both terms are 0
+            const float x = F.sig[c][min(k, nS - 1)];
+            const float tw = k < nS ? dis_r(x, true, mub, muw, rvar2) : 0.f;
+            const float tb = k < nS ? dis_r(x, false, mub, muw, rvar2) : 0.f;
+            uint32_t bits[kMaxBankIds / 32];
+#pragma unroll
+            for (int q = 0; q < kMaxBankIds / 32; ++q) bits[q] = F.black[32 * q + lane][w];
+#pragma unroll
+            for (int b = 0; b < 32; ++b) {
+                if (b % 4 == 0 && 32 * w + b >= nS) break;
+                const float aw = __shfl_sync(0xffffffffu, tw, b), ab = __shfl_sync(0xffffffffu, tb, b);
+#pragma unroll
+                for (int q = 0; q < kMaxBankIds / 32; ++q) dist[q] += (bits[q] & (1u << b)) ? ab : aw;
             }
         }
-        // dis()'s division by 2 var: a float quotient through the double
-        // reciprocal is correctly rounded for a normal result (its relative
-        // error, 2^-52, is below the 2^-49 that separates a quotient of floats
-        // from a float rounding midpoint), so each term is the IEEE quotient.
-        const double rvar2 = 1.0 / double(2.0f * var);
-        const float stepX = (1.f - ip.beginSig) / (float(nS) - 1.f);
         // std::map<float, id> keeps, for equal keys, the id inserted last: the
         // winner is the largest v, ties to the largest id.  v >= 0, so its bit
         // pattern orders like the value; (bits << 32 | id) orders like the map.
         unsigned long long best = 0ull;
-        for (int base = 0; base < ip.nIds; base += 32) {
-            const int idc = base + lane;
-            unsigned long long key = 0ull;
-            if (idc < ip.nIds) {
-                // this lane's bank row (1 / ratio), padded with +inf
-                float inv[kMaxBankRatios];
 #pragma unroll
-                for (int r = 0; r < kMaxBankRatios; ++r)
-                    inv[r] = r < ip.nRatios ? __ldg(&bankInv[idc * kMaxBankRatios + r]) : FLT_MAX;
-                float x = ip.beginSig, dist = 0.f;
-#pragma unroll 4
-                for (int k = 0; k < nS; ++k) {
-                    int ldum = 0;
-#pragma unroll
-                    for (int r = 0; r < kMaxBankRatios; ++r) ldum += (inv[r] <= x) ? 1 : 0;
-                    dist += dis_r(sg[k], (ldum & 1) == 0, mub, muw, rvar2);
-                    x += stepX;
-                }
-                const float v = expf(-dist);
-                key = (static_cast<unsigned long long>(__float_as_uint(v)) << 32) | unsigned(idc);
-            }
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                const unsigned long long ok = __shfl_xor_sync(0xffffffffu, key, o);
-                key = ok > key ? ok : key;
-            }
-            best = key > best ? key : best;
+        for (int q = 0; q < kMaxBankIds / 32; ++q) {
+            const int idc = 32 * q + lane;
+            const float v = expf(-dist[q]);
+            const unsigned long long key = (static_cast<unsigned long long>(__float_as_uint(v)) << 32) | unsigned(idc);
+            if (idc < ip.nIds && key > best) best = key;
         }
-        const int bestId = int(best & 0xffffffffull);
-        const float bestV = __uint_as_float(unsigned(best >> 32));
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const unsigned long long ok = __shfl_xor_sync(0xffffffffu, best, o);
+            best = ok > best ? ok : best;
+        }
         if (lane == 0) {
-            S.winner[c] = bestId;
-            S.vwin[c] = bestV;
+            Shared* first = &S;
+            if constexpr (CLUSTER) first = cg::this_cluster().map_shared_rank(&S, 0);
+            first->winner[c] = int(best & 0xffffffffull);
+            first->vwin[c] = __uint_as_float(unsigned(best >> 32));
         }
     }
-    __syncthreads();
-    if (tid == 0) {
+    if constexpr (CLUSTER) {
+        cg::this_cluster().sync();
+        if (crank != 0) return;
+    } else {
+        __syncthreads();
+    }
+    if (warp == 0) {
         // ID vote (Identification.cpp:1408-1431): most-voted id (first on ties),
-        // score = mean probability of its votes.
-        int counts[kMaxBankIds];
-        for (int i = 0; i < ip.nIds; ++i) counts[i] = 0;
-        for (int c = 0; c < T.ncuts; ++c)
-            if ((valid >> c) & 1u) counts[S.winner[c]]++;
-        int iMax = 0, maxSize = 0;
-        for (int i = 0; i < ip.nIds; ++i)
-            if (counts[i] > maxSize) {
-                iMax = i;
-                maxSize = counts[i];
-            }
-        float score = 0.f;
-        for (int c = 0; c < T.ncuts; ++c)
-            if (((valid >> c) & 1u) && S.winner[c] == iMax) score += S.vwin[c];
-        score /= float(maxSize);
+        // score = mean probability of its votes; a lane per cut.
+        const bool votes = lane < T.ncuts && ((valid >> lane) & 1u);
+        const int own = votes ? S.winner[lane] : -1;
+        const int n = __popc(__match_any_sync(0xffffffffu, own));
+        // the largest count, then the least id
+        unsigned key = votes ? (unsigned(n) << 16) | unsigned(0xffff - own) : 0u;
+        key = __reduce_max_sync(0xffffffffu, key);
+        const int iMax = key ? 0xffff - int(key & 0xffffu) : 0;
+        const int maxSize = int(key >> 16);
         float vmin = FLT_MAX, vmax = -FLT_MAX;
-        for (int k = 0; k < nS; ++k) {
-            vmin = fminf(vmin, S.barcode[k]);
-            vmax = fmaxf(vmax, S.barcode[k]);
+        for (int k = lane; k < nS; k += 32) {
+            vmin = fminf(vmin, F.barcode[k]);
+            vmax = fmaxf(vmax, F.barcode[k]);
         }
-        const float residual = sqrtf(S.minRes) / (vmax - vmin);
-        R.x = S.cx;
-        R.y = S.cy;
-        for (int k = 0; k < 9; ++k) R.H[k] = S.Hopt[k];
-        R.residual = residual;
-        R.nvalid = nValid;
-        R.iterations = S.iterations;
-        if (residual > 2.7f || !(residual == residual)) {
-            R.status = CCTAGB_OPTI_HAS_DIVERGED;
-            R.id = -1;
-            R.score = 0.f;
-        } else {
-            R.id = iMax;
-            R.score = score;
-            R.status = score > ip.minIdentProba ? CCTAGB_ID_RELIABLE : CCTAGB_ID_NOT_RELIABLE;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
+            vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+        }
+        if (lane == 0) {
+            float score = 0.f;
+            for (int c = 0; c < T.ncuts; ++c)
+                if (((valid >> c) & 1u) && S.winner[c] == iMax) score += S.vwin[c];
+            score /= float(maxSize);
+            const float residual = sqrtf(S.minRes) / (vmax - vmin);
+            R.x = S.cx;
+            R.y = S.cy;
+            for (int k = 0; k < 9; ++k) R.H[k] = S.Hopt[k];
+            R.residual = residual;
+            R.nvalid = nValid;
+            R.iterations = S.iterations;
+            if (residual > 2.7f || !(residual == residual)) {
+                R.status = CCTAGB_OPTI_HAS_DIVERGED;
+                R.id = -1;
+                R.score = 0.f;
+            } else {
+                R.id = iMax;
+                R.score = score;
+                R.status = score > ip.minIdentProba ? CCTAGB_ID_RELIABLE : CCTAGB_ID_NOT_RELIABLE;
+            }
         }
     }
 }
@@ -1653,7 +2000,7 @@ void upload_bank(const std::vector<std::vector<float>>& bank, float* d_bank_inv)
 }
 
 void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_tasks, IdentResult* d_res, int n,
-                     const float* d_bank_inv, const IdentParams& ip, cudaStream_t s)
+                     int maxCuts, int maxBox, const float* d_bank_inv, const IdentParams& ip, cudaStream_t s)
 {
     if (n <= 0) return;
     if (ip.gridN * ip.gridN > kMaxTrials || ip.gridN < 3 || (ip.gridN & 1) == 0)
@@ -1665,34 +2012,68 @@ void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_task
         throw Error{CCTAGB_BAD_ARG, "gnIterations must be in [1, 100]"};
     if (ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON && (ip.coarseRounds < 1 || ip.coarseRounds > 64))
         throw Error{CCTAGB_BAD_ARG, "gnCoarseRounds must be in [1, 64]"};
-    // Few markers: a cluster of blocks each, so that a launch spreads over
-    // the SMs; many (or the block layout asked for): one block each, which
-    // takes about half the SM time per marker (the per-chunk sums are the
-    // same bits).
-    int dev = 0, sms = 0;
+    // Blocks per marker and warps per block.  A round has one task per trial
+    // and chunk of 32 samples, 79 for 25 trials of 100 samples (the partial
+    // chunks packed): with few markers they spread over a cluster of 8 blocks
+    // of 10 warps, then 4 or 2 blocks of 20, as long as the markers' blocks
+    // (nearly) fit the SMs side by side: a marker's time grows with its size,
+    // so the few blocks beyond start as the smallest markers end.  With more
+    // markers a block each, of 20 warps while an SM has one marker, else two
+    // blocks of 12 warps on an SM, or for Gauss-Newton, most of whose time is
+    // serial steps of a marker, kGnBlocks of 4.  The block layout keeps to one
+    // block per marker, which takes the least SM time.
+    // Measured, against a block of 25 warps per marker (a cluster of 4 below 38
+    // markers) that read the image and one trial per warp: 28 markers of a 1080p
+    // frame 261 -> 120 us, 80 of a 3840x2160 clutter frame 588 -> 377 us, 1024
+    // candidates of 8-150 px radius 3.15 -> 1.48 ms (1.95 ms in the caller's
+    // order), by Gauss-Newton 4096 of them 2.61 -> 1.65 ms (4 to 6 blocks per SM,
+    // with room for larger markers' pixels, 3 % slower).
+    int dev = 0, sms = 0, smemBlock = 0, smemSm = 0;
     CCTAGB_CUDA(cudaGetDevice(&dev));
     CCTAGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (ip.layout != CCTAGB_IDENT_BLOCK && n * kCluster <= sms) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(unsigned(n * kCluster));
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = kCluster;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        CCTAGB_CUDA(cudaLaunchKernelEx(&cfg, k_identify<kCluster, 1>, d_img, pitch, d_tasks, d_res, d_bank_inv, ip));
-    } else if (ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON) {
-        k_identify<1, 2><<<n, kThreads, 0, s>>>(d_img, pitch, d_tasks, d_res, d_bank_inv, ip);
-        CCTAGB_CUDA(cudaGetLastError());
-    } else {
-        k_identify<1, 1><<<n, kThreads, 0, s>>>(d_img, pitch, d_tasks, d_res, d_bank_inv, ip);
-        CCTAGB_CUDA(cudaGetLastError());
-    }
+    CCTAGB_CUDA(cudaDeviceGetAttribute(&smemBlock, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    CCTAGB_CUDA(cudaDeviceGetAttribute(&smemSm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    const bool gn = ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON;
+    int cluster = 1;
+    if (ip.layout != CCTAGB_IDENT_BLOCK)
+        for (cluster = kMaxCluster; cluster > 1 && n * cluster > sms + (cluster == 2 ? sms / 4 : 0);) cluster >>= 1;
+    const int perSm = cluster > 1 || n <= sms ? 1 : gn && n > 2 * sms ? kGnBlocks : 2;
+    const int warps = cluster == kMaxCluster ? 10 : perSm == 1 ? kMaxIdWarps : perSm == 2 ? 12 : kMaxChunks;
+    // Dynamic shared memory: the lines or the Gauss-Newton samples, then the
+    // pixels of the largest marker, as far as they fit (1 KB per block is the
+    // driver's).
+    size_t work = grid_work(ip.gridN * ip.gridN, std::min(maxCuts, kMaxCuts));
+    if (gn && warps > kMaxChunks) work = std::max(work, kGnWork);
+    const size_t fixed = align16(sizeof(Shared)) + work + 1024;
+    const size_t room = std::min(size_t(smemBlock), size_t(smemSm) / size_t(perSm)) - fixed;
+    const size_t box = std::min(align16(size_t(std::max(maxBox, 0))), room & ~size_t(15));
+    const size_t smem = std::max(work + box, sizeof(FinalWork));
+    auto* kernel = cluster > 1 ? k_identify<true> : k_identify<false>;
+    CCTAGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     smemBlock - int(align16(sizeof(Shared)))));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(n * cluster));
+    cfg.blockDim = dim3(unsigned(32 * warps));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(cluster);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    CCTAGB_CUDA(cudaLaunchKernelEx(&cfg, kernel, d_img, pitch, d_tasks, d_res, d_bank_inv, ip, int(work), int(box)));
+}
+
+int ident_box(float a, float b, float angle)
+{
+    // half extents of the ellipse, and room for the margin of find_box and the
+    // rows' padding
+    const float c = std::cos(angle), s = std::sin(angle);
+    const float hx = std::sqrt(a * a * c * c + b * b * s * s), hy = std::sqrt(a * a * s * s + b * b * c * c);
+    const double w = 2.0 * hx + 20.0, h = 2.0 * hy + 10.0;
+    return w * h < double(1 << 20) ? int(w * h) : 1 << 20;  // also for NaN: as much as there is
 }
 
 void launch_cut_cost(const uint8_t* d_img, size_t pitch, const IdentTask* d_tasks, const float* d_centers,
