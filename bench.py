@@ -187,8 +187,8 @@ def stage_bytes(levels, E, S, V):
     Et, St, Vt = sum(E), sum(S), sum(V)
     return {
         "pyramid": n[0] + sum(n[1:]),                 # read level 0, write levels 1..3
-        "deriv_nms": 6 * nt,                          # 1 B in, dx+dy 4 B + class map 1 B out
-        "hyst_merge": 1 * nt,                         # class map in (tile bit planes are its own output)
+        "deriv_nms": 5 * nt + nt // 4,                # 1 B in, dx+dy 4 B and two tile bit planes out
+        "hyst_merge": nt // 4,                        # two tile bit planes in
         "hyst_compress": 3 * nt // 8,                 # two tile bit planes in, result bit plane out
         "final_thin": nt // 4,                        # result bit plane in, edge bitmap out
         "row_scan": 8 * sum(h for (_, h) in levels),

@@ -23,7 +23,6 @@ struct LevelView {
     uint8_t* src;            // W*H gray
     int16_t* dx;             // W*H
     int16_t* dy;             // W*H
-    uint8_t* map;            // W*H: 0 no edge, 1 weak candidate, 2 strong candidate
     uint32_t* hbits;         // 3 * WW*H: hysteresis planes C (candidates), R (tile-local strong closure), H (result)
     uint8_t* blab;           // uf_tiles * 128: border-position -> tile component (0xff none)
     int32_t* tcomp;          // uf_tiles * 64: union-find parents over (tile, component) ids
@@ -50,9 +49,8 @@ struct LevelView {
     int32_t* seed_votes;     // seedcap: votes the seed received
     int32_t* bigq;           // cap: points whose voter list needs a block sort
     // launch geometry of the tiled kernels
-    int nms_tx, nms_tiles;   // 30x30 output tiles
+    int dv_tx, dv_tiles;     // 64x64 derivative tiles
     int thin_tx, thin_tiles; // thinning: 32-pixel word columns x 28-row strips
-    int pix_blocks;          // 256-pixel blocks
     int uf_tx, uf_tiles;     // 32x32 hysteresis tiles
 };
 

@@ -89,11 +89,6 @@ __device__ __forceinline__ int magnitude(int16_t gx, int16_t gy)
     return int(rintf(__fsqrt_rn(__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)))));
 }
 
-__device__ __forceinline__ bool edge_bit(const LevelView& L, int x, int y)
-{
-    return (L.bitmap[size_t(y) * L.WW + (x >> 5)] >> (x & 31)) & 1u;
-}
-
 // ---------------------------------------------------------------- pyramid --
 // ImagePyramid.cpp:23-52, Level.cpp:57-81.  Exact 2x reductions (every level
 // of a frame whose sides are multiples of 8) are the rounded 2x2 mean, as
@@ -177,121 +172,234 @@ __global__ void k_resize_level(const uint8_t* __restrict__ src, int sw, int sh, 
     dst[size_t(y) * dw + x] = uint8_t(min(255, max(0, v)));
 }
 
-// --------------------------------------------- derivatives + magnitude + NMS --
-// Output tile 30x30.  Derivatives are computed on the 32x32 region around it
-// (NMS needs the magnitude of the 8 neighbours) from a 40x40 source region.
-// Thread t owns derivative column t&31 and the 8-row strip t>>5: it walks the
-// 16 source rows of its strip once and feeds each loaded row to every output
-// row whose 9x9 window covers it, which keeps each pixel's taps in the
-// reference's row-major order.
-constexpr int kNmsT = 30;      // output tile side
-constexpr int kNmsD = 32;      // derivative region side
-constexpr int kNmsS = 40;      // source region side
+// ------------------------------------------------------------- derivatives --
+// dx and dy of every level: cv::filter2D's FP32 sums over the 72 nonzero taps in
+// row-major order, rounded to int16.  The kernel is the outer product of a
+// smoothing column G (G[4] = 1) and an antisymmetric row D, up to the last
+// digits of its printed constants, so the sums are first formed separably, with
+// exact integer sums and differences of the symmetric taps, 35 operations a
+// pixel instead of 144.  That value and the reference's chain differ by less
+// than kDerivErr, so where it is further than that from a rounding boundary
+// both round to the same integer; the other pixels (0.3 % on noisy frames) are
+// listed and their chains evaluated as written.
+//
+// kDerivErr, for pixels in [0, 255] and with u = 2^-24: a rounding adds at most
+// u times its result.  The chain's partial sums (bounded by 255 times the larger
+// of their positive and negative weights) add up to 4.1e-4 for dx and 4.9e-4 for
+// dy; the separable form's row sums, bounded by 74 and 639, and their weighted
+// sums by 186, to 1.1e-4 and 1.7e-4; the factors' products differ from the
+// constants by 2.2e-6 in all.
+//
+// A warp takes 64 columns (two per lane) and kDvRows rows, walking down with the
+// last nine row sums in registers; products and sums of the two columns go in
+// pairs (fma.rn.f32x2).  Four columns per lane need fewer loads but 138
+// registers: 10 warps on an SM, which left it waiting for the tile's loads
+// (3840x2160 frame and its pyramid: 88 us; two columns 52 us; the chains for
+// every pixel, with the suppression in the same kernel, 145 us).
+constexpr float kDerivErr = 7.5e-4f;
+constexpr int kDvCols = 64, kDvWarps = 4, kDvRows = 16;
+constexpr int kDvTileRows = kDvWarps * kDvRows;
+constexpr int kDvPitch = kDvCols + 8;
+constexpr int kDvList = 512;  // unsure pixels listed per tile; above that the whole tile is redone
 
-__global__ void __launch_bounds__(128) k_deriv_nms(Levels lv, VoteParamsDev vp, int write_derivs)
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair2(float lo, float hi)
 {
-    __shared__ float s_src[kNmsS][kNmsS];
-    __shared__ int16_t s_dx[kNmsD][kNmsD];
-    __shared__ int16_t s_dy[kNmsD][kNmsD];
-    __shared__ int s_mag[kNmsD][kNmsD + 1];
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void split2(f32x2 v, float& lo, float& hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 
+// The reference's chains for the pixel whose 9x9 window starts at s.
+__device__ __noinline__ void deriv_chain(const float* s, float& ax, float& ay)
+{
+    ax = ay = 0.f;
+#pragma unroll 1
+    for (int i = 0; i < 9; ++i)
+#pragma unroll
+        for (int j = 0; j < 9; ++j) {
+            const float v = s[i * kDvPitch + j];
+            if (j != 4) ax = __fmaf_rn(cK[i][j], v, ax);
+            if (i != 4) ay = __fmaf_rn(cK[j][i], v, ay);
+        }
+}
+
+__global__ void __launch_bounds__(32 * kDvWarps) k_derivs(Levels lv)
+{
+    __shared__ __align__(16) float s_src[kDvTileRows + 8][kDvPitch];
+    __shared__ uint16_t s_list[kDvList];
+    __shared__ int s_unsure;
     int tile;
-    const int l = level_of_block(lv, blockIdx.x, &LevelView::nms_tiles, tile);
+    const int l = level_of_block(lv, blockIdx.x, &LevelView::dv_tiles, tile);
     const LevelView& L = lv.l[l];
     const int W = L.W, H = L.H;
-    const int x0 = (tile % L.nms_tx) * kNmsT;
-    const int y0 = (tile / L.nms_tx) * kNmsT;
-    const int t = threadIdx.x;
-
-    if (write_derivs) {
-        for (int i = t; i < kNmsS * kNmsS; i += 128) {
-            const int sr = i / kNmsS, sc = i % kNmsS;
-            const int yy = min(H - 1, max(0, y0 - 5 + sr));
-            const int xx = min(W - 1, max(0, x0 - 5 + sc));
-            s_src[sr][sc] = float(L.src[size_t(yy) * W + xx]);
-        }
-        __syncthreads();
-        const int c = t & 31;
-        const int r0 = (t >> 5) * 8;
-        float ax[8], ay[8];
+    const int x0 = (tile % L.dv_tx) * kDvCols, y0 = (tile / L.dv_tx) * kDvTileRows;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t == 0) s_unsure = 0;
+    if (blockIdx.x == 0)  // the counters of the launch's levels start at 0
+        for (int i = t; i < lv.n * int(sizeof(LevelCounters) / 4); i += 32 * kDvWarps)
+            reinterpret_cast<int32_t*>(lv.cnt)[i] = 0;
+    // the tile with its halo of 4, the image's border pixels repeated; inside
+    // the image and on word boundaries a word at a time, several in flight
+    constexpr int kWords = kDvPitch / 4, kStage = (kDvTileRows + 8) * kWords;
+    auto put = [&](int i, uint32_t v) {
+        const int r = i / kWords, q = i - r * kWords;
+        *reinterpret_cast<float4*>(&s_src[r][4 * q]) =
+            make_float4(float(v & 0xffu), float((v >> 8) & 0xffu), float((v >> 16) & 0xffu), float(v >> 24));
+    };
+    auto row_of = [&](int i) { return L.src + size_t(min(H - 1, max(0, y0 - 4 + i / kWords))) * W; };
+    if (x0 >= 4 && x0 + kDvCols + 4 <= W && W % 4 == 0 && (reinterpret_cast<size_t>(L.src) & 3) == 0) {
+        constexpr int kAhead = 6;
+        for (int i0 = t; i0 < kStage; i0 += kAhead * 32 * kDvWarps) {
+            uint32_t v[kAhead];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) { ax[r] = 0.f; ay[r] = 0.f; }
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            float v[9];
-#pragma unroll
-            for (int j = 0; j < 9; ++j) v[j] = s_src[r0 + q][c + j];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int i = q - r;
-                if (i < 0 || i > 8) continue;
-#pragma unroll
-                for (int j = 0; j < 9; ++j) {
-                    if (j != 4) ax[r] = __fmaf_rn(cK[i][j], v[j], ax[r]);
-                    if (i != 4) ay[r] = __fmaf_rn(cK[j][i], v[j], ay[r]);
-                }
+            for (int k = 0; k < kAhead; ++k) {
+                const int i = i0 + k * 32 * kDvWarps;
+                if (i < kStage)
+                    v[k] = __ldg(reinterpret_cast<const uint32_t*>(row_of(i) + x0 - 4 + 4 * (i % kWords)));
             }
-        }
-        // derivatives and magnitude of this thread's 8 pixels
-        const int xx = x0 - 1 + c;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int16_t gx = sat_round16(ax[r]), gy = sat_round16(ay[r]);
-            s_dx[r0 + r][c] = gx;
-            s_dy[r0 + r][c] = gy;
-            const int yy = y0 - 1 + r0 + r;
-            s_mag[r0 + r][c] = xx >= 0 && xx < W && yy >= 0 && yy < H ? magnitude(gx, gy) : 0;
+            for (int k = 0; k < kAhead; ++k)
+                if (i0 + k * 32 * kDvWarps < kStage) put(i0 + k * 32 * kDvWarps, v[k]);
         }
     } else {
-        // Derivatives supplied by the caller: load them with the same halo.
-        for (int i = t; i < kNmsD * kNmsD; i += 128) {
-            const int r = i / kNmsD, c = i % kNmsD;
-            const int yy = y0 - 1 + r, xx = x0 - 1 + c;
-            int16_t gx = 0, gy = 0;
-            if (xx >= 0 && xx < W && yy >= 0 && yy < H) {
-                gx = L.dx[size_t(yy) * W + xx];
-                gy = L.dy[size_t(yy) * W + xx];
+        constexpr int kAhead = 3;
+        for (int i0 = t; i0 < kStage; i0 += kAhead * 32 * kDvWarps) {
+            uint32_t v[kAhead][4];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                const int i = min(i0 + k * 32 * kDvWarps, kStage - 1);
+                const uint8_t* row = row_of(i);
+                const int x = x0 - 4 + 4 * (i % kWords);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[k][q] = __ldg(row + min(W - 1, max(0, x + q)));
             }
-            s_dx[r][c] = gx;
-            s_dy[r][c] = gy;
-            s_mag[r][c] = xx >= 0 && xx < W && yy >= 0 && yy < H ? magnitude(gx, gy) : 0;
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k)
+                if (i0 + k * 32 * kDvWarps < kStage)
+                    put(i0 + k * 32 * kDvWarps, v[k][0] | v[k][1] << 8 | v[k][2] << 16 | v[k][3] << 24);
         }
     }
     __syncthreads();
-    // NMS, cvRecode.cpp:258-323: lane ox of warp w takes column ox of rows
-    // w, w + 4, ...
-    const int TG22 = int(0.4142135623730950488016887242097 * (1 << 15) + 0.5);
-    const int ox = t & 31;
-    for (int oy = t >> 5; oy < kNmsT; oy += 4) {
-        const int x = x0 + ox, y = y0 + oy;
-        if (ox >= kNmsT || x >= W || y >= H) continue;
-        const int r = oy + 1, c = ox + 1;
-        int gx = s_dx[r][c], gy = s_dy[r][c];
-        const int s = gx ^ gy;
-        const int m = s_mag[r][c];
-        gx = abs(gx);
-        gy = abs(gy);
-        bool is_max = false;
-        if (m > vp.low) {
-            const int tg22x = gx * TG22;
-            const int tg67x = tg22x + ((gx + gx) << 15);
-            const int gy15 = gy << 15;
-            if (gy15 < tg22x) {
-                is_max = m > s_mag[r][c - 1] && m >= s_mag[r][c + 1];
-            } else if (gy15 > tg67x) {
-                is_max = m > s_mag[r - 1][c] && m >= s_mag[r + 1][c];
+    // D[8 - j] and G[j], j = 0..3 (cK's center row, and its columns over it)
+    const float D[4] = {0.000427124283626f, 0.010608310271112f, 0.086157117207395f, 0.193064705260108f};
+    const float G[4] = {0.000335462624f, 0.0111089963f, 0.135335281f, 0.606530666f};
+    f32x2 D2[4], G2[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        D2[j] = pair2(D[j], D[j]);
+        G2[j] = pair2(G[j], G[j]);
+    }
+    const f32x2 magic = pair2(12582912.f, 12582912.f), nmagic = pair2(-12582912.f, -12582912.f);
+    const f32x2 minus1 = pair2(-1.f, -1.f);
+    f32x2 wd[9], wg[9];  // the last nine rows' sums (slot = row mod 9)
+    const int yw = y0 + warp * kDvRows;
+    const int rows = min(kDvRows, H - yw) + 8;
+    // four-byte stores where the rows (and the caller's planes) allow them
+    const bool wide = W % 2 == 0 && ((reinterpret_cast<size_t>(L.dx) | reinterpret_cast<size_t>(L.dy)) & 3) == 0;
+    const int xq = x0 + 2 * lane;
+    for (int r9 = 0; r9 < rows; r9 += 9) {
+#pragma unroll
+        for (int u = 0; u < 9; ++u) {
+            const int r = r9 + u;
+            if (r >= rows) break;
+            const float2* p = reinterpret_cast<const float2*>(&s_src[warp * kDvRows + r][2 * lane]);
+            float v[10];
+#pragma unroll
+            for (int j = 0; j < 5; ++j) {
+                const float2 q = p[j];
+                v[2 * j] = q.x;
+                v[2 * j + 1] = q.y;
+            }
+            f32x2 d = 0, g = pair2(v[4], v[5]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const f32x2 df = pair2(v[8 - j] - v[j], v[9 - j] - v[1 + j]);
+                const f32x2 sm = pair2(v[8 - j] + v[j], v[9 - j] + v[1 + j]);
+                d = j == 0 ? mul2(D2[0], df) : fma2(D2[j], df, d);
+                g = fma2(G2[j], sm, g);
+            }
+            wd[u] = d;
+            wg[u] = g;
+            if (r < 8) continue;
+            // output row r - 8: slots u + 1 .. u + 9 (mod 9) hold its nine rows
+            f32x2 x = wd[(u + 5) % 9], y = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int a = (u + 1 + j) % 9, b = (u + 9 - j) % 9;
+                x = fma2(G2[j], add2(wd[a], wd[b]), x);
+                const f32x2 df = fma2(minus1, wg[a], wg[b]);
+                y = j == 0 ? mul2(D2[0], df) : fma2(D2[j], df, y);
+            }
+            // rounded to the nearest integer (in the low bits of the sum with
+            // 1.5 * 2^23), and the distance to it
+            const f32x2 mx = add2(x, magic), my = add2(y, magic);
+            const f32x2 ex = fma2(minus1, add2(mx, nmagic), x), ey = fma2(minus1, add2(my, nmagic), y);
+            const uint32_t ox = __byte_perm(uint32_t(mx), uint32_t(mx >> 32), 0x5410);
+            const uint32_t oy = __byte_perm(uint32_t(my), uint32_t(my >> 32), 0x5410);
+            float a0, a1, b0, b1;
+            split2(ex, a0, a1);
+            split2(ey, b0, b1);
+            const int yo = yw + r - 8;
+            const size_t o = size_t(yo) * W + xq;
+            if (wide) {
+                if (xq < W) {
+                    *reinterpret_cast<uint32_t*>(L.dx + o) = ox;
+                    *reinterpret_cast<uint32_t*>(L.dy + o) = oy;
+                }
             } else {
-                const int sg = s < 0 ? -1 : 1;
-                is_max = m > s_mag[r - 1][c - sg] && m > s_mag[r + 1][c + sg];
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if (xq + k < W) {
+                        L.dx[o + k] = int16_t(ox >> (16 * k));
+                        L.dy[o + k] = int16_t(oy >> (16 * k));
+                    }
+            }
+            const float w0 = fmaxf(fabsf(a0), fabsf(b0)), w1 = fmaxf(fabsf(a1), fabsf(b1));
+            if (fmaxf(w0, w1) > 0.5f - kDerivErr) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if ((k ? w1 : w0) > 0.5f - kDerivErr && xq + k < W) {
+                        const int i = atomicAdd(&s_unsure, 1);
+                        if (i < kDvList) s_list[i] = uint16_t((yo - y0) * kDvCols + 2 * lane + k);
+                    }
             }
         }
-        const size_t p = size_t(y) * W + x;
-        const uint8_t cls = is_max ? (m > vp.high ? 2 : 1) : 0;
-        L.map[p] = cls;
-        if (write_derivs) {
-            L.dx[p] = s_dx[r][c];
-            L.dy[p] = s_dy[r][c];
-        }
+    }
+    __syncthreads();  // and the stores above come before those below
+    const bool all = s_unsure > kDvList;
+    const int n = all ? kDvTileRows * kDvCols : s_unsure;
+    for (int i = t; i < n; i += 32 * kDvWarps) {
+        const int p = all ? i : s_list[i];
+        const int r = p / kDvCols, c = p % kDvCols;
+        if (x0 + c >= W || y0 + r >= H) continue;
+        float ax, ay;
+        deriv_chain(&s_src[r][c], ax, ay);
+        const size_t o = size_t(y0 + r) * W + x0 + c;
+        L.dx[o] = sat_round16(ax);
+        L.dy[o] = sat_round16(ay);
     }
 }
 
@@ -300,14 +408,14 @@ __global__ void __launch_bounds__(128) k_deriv_nms(Levels lv, VoteParamsDev vp, 
 // 8-connected components of NMS candidates that contain a strong pixel.  Here
 // the image is cut into 32x32 tiles, one warp each, lane r holding row r of
 // the tile as 32-bit masks (candidates C, strong S):
-//  1. k_hyst_tiles: the closure of S within C inside the tile (R, bit-parallel
-//     dilation: rows shifted by one bit, neighbour rows by shuffles), and the
-//     components that touch the tile border, one flood fill each, labelled
-//     per border position, with whether they hold a strong pixel;
-//  2. k_hyst_unions / k_hyst_roots: those border components joined across
+//  1. k_nms_tiles: non-maximum suppression (C, S), the closure R of S within C
+//     inside the tile, and the other components of C that touch the tile border,
+//     labelled per border position;
+//  2. k_hyst_unions / k_hyst_roots: those weak border components joined across
 //     tile borders by a lock-free union-find over (tile, component) ids
 //     (parent <= self, roots linked by atomicMin, so any schedule gives the
-//     same sets), and each set marked strong at its root if a member is;
+//     same sets) or marked where they meet a pixel of R, and each set with a
+//     marked member marked strong at its root;
 //  3. k_hyst_final: per tile, R plus the border pixels of strong sets, closed
 //     within C again: the hysteresis result H, one bit per pixel.
 // A pixel is in H exactly when its component holds a strong pixel: a path to
@@ -332,8 +440,14 @@ __device__ __forceinline__ int uf_find(const int32_t* L, int p)
 __device__ __forceinline__ void uf_union(int32_t* L, int a, int b, int32_t* err)
 {
     for (int it = 0; it < kUfCap; ++it) {
-        a = uf_find(L, a);
-        b = uf_find(L, b);
+        // both walks to the roots side by side
+        int pa = *(volatile const int32_t*)&L[a], pb = *(volatile const int32_t*)&L[b];
+        for (int guard = 0; (pa != a || pb != b) && guard < kUfCap; ++guard) {
+            a = pa;
+            b = pb;
+            pa = *(volatile const int32_t*)&L[a];
+            pb = *(volatile const int32_t*)&L[b];
+        }
         if (a == b) return;
         if (a > b) { const int tmp = a; a = b; b = tmp; }
         const int old = atomicMin(&L[b], a);
@@ -344,10 +458,14 @@ __device__ __forceinline__ void uf_union(int32_t* L, int a, int b, int32_t* err)
 }
 
 // The closure of `seed` (a subset of c) within c, 8-connected, over the
-// warp's tile (lane = row).  Each round adds a pixel or ends the loop, so it
-// ends within the tile's 1024 pixels.
+// warp's tile (lane = row).  A round takes the neighbour rows' pixels and goes
+// on along the row's runs: upwards to their ends (adding pixels of a run to it
+// carries through it), downwards seven pixels (c2: pixels whose lower neighbour
+// is one too, c4: whose three lower neighbours are).  Each round adds a pixel or
+// ends the loop, so it ends within the tile's 1024 pixels.
 __device__ __forceinline__ uint32_t tile_closure(uint32_t seed, uint32_t c, int lane)
 {
+    const uint32_t c2 = c & (c >> 1), c4 = c2 & (c2 >> 2);
     uint32_t r = seed & c;
     for (int it = 0; it <= kTile * kTile; ++it) {
         uint32_t up = __shfl_up_sync(0xffffffffu, r, 1);
@@ -355,7 +473,10 @@ __device__ __forceinline__ uint32_t tile_closure(uint32_t seed, uint32_t c, int 
         if (lane == 0) up = 0u;
         if (lane == kTile - 1) dn = 0u;
         const uint32_t v = r | up | dn;
-        const uint32_t nb = (v | (v << 1) | (v >> 1)) & c;
+        uint32_t nb = (v | (v << 1) | (v >> 1)) & c;
+        nb |= ((nb + c) ^ c) & c;
+        nb |= c2 & (nb >> 2);
+        nb |= c4 & (nb >> 4);
         if (!__any_sync(0xffffffffu, nb != r)) break;
         r = nb;
     }
@@ -391,117 +512,293 @@ __device__ __forceinline__ uint32_t* plane_h(const LevelView& L) { return L.hbit
 
 constexpr int kHystWarps = 4;
 
-__global__ void __launch_bounds__(32 * kHystWarps) k_hyst_tiles(Levels lv, int total_tiles)
+// Magnitude and direction of a pixel as the suppression reads them.  GIVEN:
+// derivatives of any size (the caller's), in the reference's own arithmetic;
+// else those of k_derivs, whose magnitude is below 263: their squares' sum is
+// exact and its root is never near a half, so the approximate root rounds to
+// the same integer, and the direction tests are exact in floats.
+template <bool GIVEN>
+struct Gradient {
+    float m;     // magnitude, an integer
+    int sector;  // 0 horizontal, 1 vertical, 2 and 3 the diagonals (signs equal, different)
+};
+template <bool GIVEN>
+__device__ __forceinline__ Gradient<GIVEN> gradient_of(int gx, int gy)
 {
-    __shared__ uint8_t s_lab[kHystWarps][kBorderPos];
+    Gradient<GIVEN> g;
+    const int diag = (gx ^ gy) < 0 ? 3 : 2;
+    if (GIVEN) {
+        g.m = float(magnitude(int16_t(gx), int16_t(gy)));
+        const int TG22 = int(0.4142135623730950488016887242097 * (1 << 15) + 0.5);
+        const unsigned ax = unsigned(abs(gx)), ay = unsigned(abs(gy));
+        const int tg22x = int(ax * unsigned(TG22));
+        const int tg67x = int(unsigned(tg22x) + ((ax + ax) << 15));
+        const int gy15 = int(ay << 15);
+        g.sector = gy15 < tg22x ? 0 : gy15 > tg67x ? 1 : diag;
+    } else {
+        // small integers to floats through the bits of 1.5 * 2^23 + n
+        const float fx = fabsf(__fsub_rn(__int_as_float(0x4B400000 + gx), 12582912.f));
+        const float fy = fabsf(__fsub_rn(__int_as_float(0x4B400000 + gy), 12582912.f));
+        float r;
+        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fmaf_rn(fx, fx, __fmul_rn(fy, fy))));
+        g.m = __fsub_rn(__fadd_rn(r, 12582912.f), 12582912.f);
+        // TG22 = 13573 = tan(22.5 deg) * 2^15; tan(67.5 deg) = tan(22.5 deg) + 2
+        const float y15 = __fmul_rn(fy, 32768.f);
+        g.sector = y15 < __fmul_rn(fx, 13573.f) ? 0 : y15 > __fmul_rn(fx, 13573.f + 65536.f) ? 1 : diag;
+    }
+    return g;
+}
+
+// Non-maximum suppression (cvRecode.cpp:258-323) and step 1 of the hysteresis,
+// a block of WARPS warps per tile: each suppresses its rows (lane = column),
+// then all hold the tile's masks (lane = row).  The pixels of R need no
+// component: what they touch across the border is strong.  So only the weak
+// components that touch the border are flooded, one by one, in rounds that fill
+// runs of a row, each warp from its sides of the tile; a component's label is
+// its first border position, the same from every side, numbered at the end.
+// A tile is one long chain of instructions: with few tiles four warps shorten
+// it, with many one warp takes fewer instructions in all.  Measured, one warp
+// and four (suppression included): 640x480 21 and 10 us, 1080p and its pyramid
+// (2,725 tiles) 33 and 31 us, 3840x2160 clutter 85 and 98 us, sixteen 1080p
+// frames 315 and 432 us.  With a flood per border component, strong ones too, a
+// pixel per round, the hysteresis alone took 22 us of the small frame, 26 of the
+// 1080p frame; a union-find over the runs of the tile 35 us and 58 us.
+constexpr int kNmsFewTiles = 148 * 20;
+
+template <bool GIVEN, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) k_nms_tiles(Levels lv, VoteParamsDev vp)
+{
+    constexpr int kRows = kTile / WARPS;             // of a warp
+    constexpr int kGroup = WARPS == 4 ? kRows + 2 : 8;  // rows whose loads are in flight together
+    static_assert(WARPS == 4 || WARPS == 1, "sides of the tile per warp");
+    __shared__ float s_side[WARPS][2][kRows + 2];  // magnitudes left and right of the tile
+    __shared__ uint32_t s_c[kTile], s_st[kTile];
+    __shared__ uint8_t s_lab[kBorderPos], s_rank[kBorderPos];
+    const unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = blockIdx.x * kHystWarps + warp;
-    if (g >= total_tiles) return;
     int tile;
-    const int l = level_of_tile(lv, g, tile);
+    const int l = level_of_block(lv, blockIdx.x, &LevelView::uf_tiles, tile);
     const LevelView& L = lv.l[l];
+    const int W = L.W, H = L.H;
     const int tx = tile % L.uf_tx, ty = tile / L.uf_tx;
     const int x0 = tx * kTile, y0 = ty * kTile;
-    const int rows = min(kTile, L.H - y0), cols = min(kTile, L.W - x0);
-    // row masks of the tile: lane r keeps row r
-    uint32_t c = 0u, st = 0u;
-#pragma unroll 4
-    for (int r = 0; r < kTile; ++r) {
-        uint8_t v = 0;
-        if (r < rows && lane < cols) v = L.map[size_t(y0 + r) * L.W + x0 + lane];
-        const uint32_t cm = __ballot_sync(0xffffffffu, v != 0), sm = __ballot_sync(0xffffffffu, v == 2);
-        if (lane == r) {
-            c = cm;
-            st = sm;
+    const int rows = min(kTile, H - y0), cols = min(kTile, W - x0);
+    const int yw = y0 + warp * kRows - 1;  // the first of the warp's rows, with one above and below
+    for (int i = lane; i < 2 * (kRows + 2); i += 32) {
+        const int side = i >= kRows + 2 ? 1 : 0, r = i - side * (kRows + 2);
+        const int x = side ? x0 + kTile : x0 - 1;
+        float m = 0.f;
+        if (unsigned(yw + r) < unsigned(H) && unsigned(x) < unsigned(W)) {
+            const size_t p = size_t(yw + r) * W + x;
+            m = gradient_of<GIVEN>(L.dx[p], L.dy[p]).m;
+        }
+        s_side[warp][side][r] = m;
+    }
+    for (int i = threadIdx.x; i < kBorderPos; i += 32 * WARPS) s_lab[i] = 0xff;
+    __syncwarp();
+    float ul = 0.f, uc = 0.f, ur = 0.f, cl = 0.f, cc = 0.f, cr = 0.f;
+    int sector = 0;
+    const float low = float(vp.low), high = float(vp.high);
+    const bool in = lane < cols;
+    for (int r0 = 0; r0 < kRows + 2; r0 += kGroup) {
+        int gx[kGroup], gy[kGroup];
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) {
+            gx[u] = gy[u] = 0;
+            if (r0 + u < kRows + 2 && unsigned(yw + r0 + u) < unsigned(H) && in) {
+                const size_t p = size_t(yw + r0 + u) * W + x0 + lane;
+                gx[u] = L.dx[p];
+                gy[u] = L.dy[p];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) {
+            const int r = r0 + u;
+            if (r >= kRows + 2) break;
+            Gradient<GIVEN> q = gradient_of<GIVEN>(gx[u], gy[u]);
+            if (unsigned(yw + r) >= unsigned(H) || !in) q.m = 0.f;
+            float dl = __shfl_up_sync(kAll, q.m, 1), dr = __shfl_down_sync(kAll, q.m, 1);
+            if (lane == 0) dl = s_side[warp][0][r];
+            if (lane == kTile - 1) dr = s_side[warp][1][r];
+            if (r >= 2) {  // cvRecode.cpp:258-323 for the row above
+                const float n1 = sector == 0 ? cl : sector == 1 ? uc : sector == 2 ? ul : ur;
+                const float n2 = sector == 0 ? cr : sector == 1 ? q.m : sector == 2 ? dr : dl;
+                const int row = warp * kRows + r - 2;
+                const bool cand = in && row < rows && cc > low && cc > n1 && (sector >= 2 ? cc > n2 : cc >= n2);
+                const uint32_t cm = __ballot_sync(kAll, cand), sm = __ballot_sync(kAll, cand && cc > high);
+                if (lane == 0) {
+                    s_c[row] = cm;
+                    s_st[row] = sm;
+                }
+            }
+            ul = cl;
+            uc = cc;
+            ur = cr;
+            cl = dl;
+            cc = q.m;
+            cr = dr;
+            sector = q.sector;
         }
     }
-    const uint32_t R = tile_closure(st, c, lane);
-    if (lane < rows) {
-        const size_t w = size_t(y0 + lane) * L.WW + tx;
-        plane_c(L)[w] = c;
-        plane_r(L)[w] = R;
-    }
-    for (int i = lane; i < kBorderPos; i += 32) s_lab[warp][i] = 0xff;
-    __syncwarp();
-    // border components, one flood fill each from an unlabelled border pixel
-    const uint32_t bmask = (lane == 0 || lane == kTile - 1) ? c : (c & (1u | (1u << (kTile - 1))));
-    uint32_t unl = bmask;
-    uint64_t strong = 0ull;
-    int ncomp = 0;
-    while (__any_sync(0xffffffffu, unl != 0u)) {
-        const uint32_t have = __ballot_sync(0xffffffffu, unl != 0u);
+    __syncthreads();
+    const uint32_t c = s_c[lane];
+    const uint32_t R = tile_closure(s_st[lane], c, lane);
+    const bool firstRow = lane == 0, lastRow = lane == kTile - 1;
+    const uint32_t bmask = firstRow || lastRow ? c : c & 0x80000001u;
+    uint32_t todo = bmask & ~R;
+    if (WARPS == 4)
+        todo &= warp == 0 ? (firstRow ? ~0u : 0u) : warp == 1 ? (lastRow ? ~0u : 0u) : warp == 2 ? 1u : 0x80000000u;
+    for (unsigned have; (have = __ballot_sync(kAll, todo != 0u)) != 0u;) {
         const int sl = __ffs(have) - 1;
-        const uint32_t sb = __shfl_sync(0xffffffffu, unl & (0u - unl), sl);
-        const uint32_t m = tile_closure(lane == sl ? sb : 0u, c, lane);
-        if (ncomp >= kTileComps) {  // cannot happen (<= 62 components); flagged, not silent
-            if (lane == 0) atomicOr(&lv.cnt[l].err, kErrUnionFind);
-            break;
-        }
-        if (__any_sync(0xffffffffu, (m & R) != 0u)) strong |= 1ull << ncomp;
-        uint32_t bm = m & bmask;
-        while (bm) {
-            const int b = __ffs(bm) - 1;
-            bm &= bm - 1;
-            s_lab[warp][border_pos(b, lane)] = uint8_t(ncomp);
-        }
-        unl &= ~m;
-        ++ncomp;
+        const uint32_t m = tile_closure(lane == sl ? todo & (0u - todo) : 0u, c, lane);
+        todo &= ~m;
+        const uint32_t bm = m & bmask;
+        const int own = bm ? min(border_pos(__ffs(bm) - 1, lane), border_pos(31 - __clz(bm), lane)) : 255;
+        const int label = __reduce_min_sync(kAll, unsigned(own));
+        for (uint32_t q = bm; q; q &= q - 1) s_lab[border_pos(__ffs(q) - 1, lane)] = uint8_t(label);
     }
-    __syncwarp();
-    const size_t base = size_t(tile) * kTileComps;
-    for (int k = lane; k < kTileComps; k += 32) {
-        L.tcomp[base + k] = int32_t(base + k);
-        L.tflag[base + k] = (k < ncomp && ((strong >> k) & 1ull)) ? 1 : 0;
+    __syncthreads();
+    if (warp == 0) {
+        int n = 0;
+        for (int w = 0; w < kBorderPos / 32; ++w) {
+            const int p = 32 * w + lane;
+            const unsigned m = __ballot_sync(kAll, s_lab[p] == p);
+            s_rank[p] = uint8_t(n + __popc(m & ((1u << lane) - 1u)));
+            n += __popc(m);
+        }
+        if (n > kTileComps && lane == 0) atomicOr(&lv.cnt[l].err, kErrUnionFind);  // cannot happen (<= 62)
+        if (lane < rows) {
+            const size_t w = size_t(y0 + lane) * L.WW + tx;
+            plane_c(L)[w] = c;
+            plane_r(L)[w] = R;
+        }
     }
-    for (int i = lane; i < kBorderPos; i += 32) L.blab[size_t(tile) * kBorderPos + i] = s_lab[warp][i];
+    __syncthreads();
+    for (int p = threadIdx.x; p < kBorderPos; p += 32 * WARPS) {
+        const int lab = s_lab[p];
+        L.blab[size_t(tile) * kBorderPos + p] = lab == 0xff ? uint8_t(0xff) : s_rank[lab];
+    }
+    for (int k = threadIdx.x; k < kTileComps; k += 32 * WARPS) {
+        const size_t id = size_t(tile) * kTileComps + k;
+        L.tcomp[id] = int32_t(id);
+        L.tflag[id] = 0;
+    }
 }
 
-// The (tile, component) id of border pixel (x, y) of the level.
-__device__ __forceinline__ int border_comp(const LevelView& L, int x, int y)
-{
-    const int tile = (y / kTile) * L.uf_tx + x / kTile;
-    const int lab = L.blab[size_t(tile) * kBorderPos + border_pos(x % kTile, y % kTile)];
-    return tile * kTileComps + lab;
-}
-
-__device__ __forceinline__ bool cand_bit(const LevelView& L, int x, int y)
-{
-    return (plane_c(L)[size_t(y) * L.WW + (x >> 5)] >> (x & 31)) & 1u;
-}
-
-// Unions across tile borders: the first row of a tile with the row above
-// (three neighbours each), the first column with the column to the left.
-// Every 8-neighbour pair that straddles a tile border meets here.
+// Step 2: pairs of neighbours across tile borders, two warps per tile: its first
+// row with the row above (lane = column, three neighbours each), its first
+// column with the column to the left (lane = row).  Every 8-neighbour pair that
+// straddles a tile border meets here.  Two weak components are joined, once for
+// neighbouring pixels of the same two; a weak one next to a pixel of R is marked
+// strong.  All words and labels are loaded first, side by side: the kernel is a
+// chain of loads and atomics (17 us of a 1080p frame with each pixel's bit, then
+// its label, then its neighbours' loaded in turn and every pair joined, 11 us now).
 __global__ void __launch_bounds__(64) k_hyst_unions(Levels lv)
 {
     int tile;
     const int l = level_of_block(lv, blockIdx.x, &LevelView::uf_tiles, tile);
     const LevelView& L = lv.l[l];
-    const int x0 = (tile % L.uf_tx) * kTile, y0 = (tile / L.uf_tx) * kTile;
-    const int t = threadIdx.x;
-    const bool row = t < 32;
-    const int x = row ? x0 + t : x0, y = row ? y0 : y0 + (t - 32);
-    if (x >= L.W || y >= L.H) return;
-    if (row ? y == 0 : x == 0) return;
-    if (!cand_bit(L, x, y)) return;
-    int32_t* err = &lv.cnt[l].err;
-    const int a = border_comp(L, x, y);
-    for (int d = -1; d <= 1; ++d) {
-        const int qx = row ? x + d : x - 1, qy = row ? y - 1 : y + d;
-        if (qx < 0 || qx >= L.W || qy < 0 || qy >= L.H) continue;
-        if (qx / kTile == x / kTile && qy / kTile == y / kTile) continue;  // same tile: joined in step 1
-        if (cand_bit(L, qx, qy)) uf_union(L.tcomp, a, border_comp(L, qx, qy), err);
+    const int tx = tile % L.uf_tx, ty = tile / L.uf_tx, tilesY = L.uf_tiles / L.uf_tx;
+    const int y0 = ty * kTile;
+    const int lane = threadIdx.x & 31;
+    const bool row = threadIdx.x < 32;
+    if (row ? ty == 0 : tx == 0) return;
+    const uint32_t* C = plane_c(L);
+    const uint32_t* R = plane_r(L);
+    const uint8_t* lab = L.blab + size_t(tile) * kBorderPos;
+    auto word = [&](const uint32_t* plane, int wx, int y) {
+        return wx >= 0 && wx < L.WW && y >= 0 && y < L.H ? __ldg(plane + size_t(y) * L.WW + wx) : 0u;
+    };
+    // component at border position `pos` of the tile (dx, dy) tiles away
+    auto comp = [&](int dx, int dy, int pos) {
+        const int qx = tx + dx, qy = ty + dy;
+        if (qx < 0 || qx >= L.uf_tx || qy < 0 || qy >= tilesY) return 0;
+        const int t = tile + dy * L.uf_tx + dx;
+        return t * kTileComps + int(__ldg(L.blab + size_t(t) * kBorderPos + pos));
+    };
+    // own pixel and the three across the border: candidate, in R, component
+    bool oc, orr, nc[3], nr[3];
+    int oa, nb[3];
+    if (row) {
+        const uint32_t c0 = word(C, tx, y0), r0 = word(R, tx, y0);
+        const uint32_t um = word(C, tx - 1, y0 - 1), uc = word(C, tx, y0 - 1), up = word(C, tx + 1, y0 - 1);
+        const uint32_t sm = word(R, tx - 1, y0 - 1), sc = word(R, tx, y0 - 1), sp = word(R, tx + 1, y0 - 1);
+        const int up0 = comp(0, -1, border_pos(lane, kTile - 1));
+        const int upL = comp(-1, -1, border_pos(kTile - 1, kTile - 1)), upR = comp(1, -1, border_pos(0, kTile - 1));
+        oa = tile * kTileComps + int(__ldg(lab + border_pos(lane, 0)));
+        oc = c0 >> lane & 1u;
+        orr = r0 >> lane & 1u;
+        nc[1] = uc >> lane & 1u;
+        nr[1] = sc >> lane & 1u;
+        nb[1] = up0;
+        nc[0] = lane > 0 ? uc >> (lane - 1) & 1u : um >> 31;
+        nr[0] = lane > 0 ? sc >> (lane - 1) & 1u : sm >> 31;
+        nc[2] = lane < 31 ? uc >> (lane + 1) & 1u : up & 1u;
+        nr[2] = lane < 31 ? sc >> (lane + 1) & 1u : sp & 1u;
+        nb[0] = __shfl_up_sync(0xffffffffu, up0, 1);
+        nb[2] = __shfl_down_sync(0xffffffffu, up0, 1);
+        if (lane == 0) nb[0] = upL;
+        if (lane == 31) nb[2] = upR;
+    } else {
+        const int y = y0 + lane;
+        const uint32_t c0 = word(C, tx, y), r0 = word(R, tx, y);
+        const uint32_t lc = word(C, tx - 1, y) >> 31, lr = word(R, tx - 1, y) >> 31;
+        const uint32_t ac = word(C, tx - 1, y0 - 1) >> 31, ar = word(R, tx - 1, y0 - 1) >> 31;
+        const uint32_t dc = word(C, tx - 1, y0 + kTile) >> 31, dr = word(R, tx - 1, y0 + kTile) >> 31;
+        const int left = comp(-1, 0, border_pos(kTile - 1, lane));
+        const int above = comp(-1, -1, border_pos(kTile - 1, kTile - 1)), below = comp(-1, 1, border_pos(kTile - 1, 0));
+        oa = tile * kTileComps + int(__ldg(lab + border_pos(0, lane)));
+        oc = c0 & 1u;
+        orr = r0 & 1u;
+        nc[1] = lc;
+        nr[1] = lr;
+        nb[1] = left;
+        const uint32_t uc = __shfl_up_sync(0xffffffffu, lc, 1), ur = __shfl_up_sync(0xffffffffu, lr, 1);
+        const uint32_t wc = __shfl_down_sync(0xffffffffu, lc, 1), wr = __shfl_down_sync(0xffffffffu, lr, 1);
+        nb[0] = __shfl_up_sync(0xffffffffu, left, 1);
+        nb[2] = __shfl_down_sync(0xffffffffu, left, 1);
+        nc[0] = lane > 0 ? uc : ac;
+        nr[0] = lane > 0 ? ur : ar;
+        nc[2] = lane < 31 ? wc : dc;
+        nr[2] = lane < 31 ? wr : dr;
+        if (lane == 0) nb[0] = above;
+        if (lane == 31) nb[2] = below;
     }
+    // weak-weak pairs, without those this lane or the one before has already
+    bool join[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        join[d] = false;
+        if (!oc || !nc[d] || (orr && nr[d])) continue;
+        if (orr) L.tflag[nb[d]] = 1;
+        else if (nr[d]) L.tflag[oa] = 1;
+        else join[d] = true;
+    }
+    join[0] = join[0] && !(join[1] && nb[0] == nb[1]);
+    join[2] = join[2] && !(join[1] && nb[2] == nb[1]) && !(join[0] && nb[2] == nb[0]);
+    const int pa = __shfl_up_sync(0xffffffffu, join[1] ? oa : -1, 1), pb = __shfl_up_sync(0xffffffffu, nb[1], 1);
+    if (lane > 0 && pa == oa && pb == nb[1]) join[1] = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        if (join[d]) uf_union(L.tcomp, oa, nb[d], &lv.cnt[l].err);
 }
 
-// Each set with a strong member is marked strong at its root.
-__global__ void __launch_bounds__(kTileComps) k_hyst_roots(Levels lv)
+// Each set with a marked member is marked strong at its root; four components
+// per thread.
+__global__ void __launch_bounds__(256) k_hyst_roots(Levels lv, int total_tiles)
 {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int kPer = kTileComps / 4;  // threads per tile
+    if (i >= total_tiles * kPer) return;
     int tile;
-    const int l = level_of_block(lv, blockIdx.x, &LevelView::uf_tiles, tile);
+    const int l = level_of_tile(lv, i / kPer, tile);
     const LevelView& L = lv.l[l];
-    const int id = tile * kTileComps + threadIdx.x;
-    if (L.tflag[id] & 1) atomicOr(&L.tflag[uf_find(L.tcomp, id)], 2);
+    const int id = tile * kTileComps + 4 * (i % kPer);
+    const int4 f = *reinterpret_cast<const int4*>(L.tflag + id);
+    const int own[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (own[k] & 1) atomicOr(&L.tflag[uf_find(L.tcomp, id + k)], 2);
 }
 
 __global__ void __launch_bounds__(32 * kHystWarps) k_hyst_final(Levels lv, int total_tiles)
@@ -620,7 +917,7 @@ __global__ void __launch_bounds__(32 * kThinWarps) k_final_thin(Levels lv, int t
     if (lane >= 2 && lane < 2 + kThinRows && y < H) {
         const uint32_t word = uint32_t(out >> 16);
         L.bitmap[size_t(y) * WW + wx] = word;
-        if (word) atomicAdd(&L.row_count[y], __popc(word));
+        if (word && L.row_count) atomicAdd(&L.row_count[y], __popc(word));
     }
 }
 
@@ -1382,14 +1679,20 @@ int launch_pack(const PackSegs& p, int32_t* dst, cudaStream_t s)
 static void launch_edges(const Levels& lv, const VoteParamsDev& vp, cudaStream_t s, int write_derivs,
                          cudaEvent_t* ev)
 {
-    k_deriv_nms<<<total_of(lv, &LevelView::nms_tiles), 128, 0, s>>>(lv, vp, write_derivs);
-    mark(ev, kStDerivNms + 1, s);
     const int tiles = total_of(lv, &LevelView::uf_tiles);
     const int hb = (tiles + kHystWarps - 1) / kHystWarps;
-    k_hyst_tiles<<<hb, 32 * kHystWarps, 0, s>>>(lv, tiles);
+    if (write_derivs) {
+        k_derivs<<<total_of(lv, &LevelView::dv_tiles), 32 * kDvWarps, 0, s>>>(lv);
+        if (tiles <= kNmsFewTiles) k_nms_tiles<false, 4><<<tiles, 128, 0, s>>>(lv, vp);
+        else k_nms_tiles<false, 1><<<tiles, 32, 0, s>>>(lv, vp);
+    } else {
+        if (tiles <= kNmsFewTiles) k_nms_tiles<true, 4><<<tiles, 128, 0, s>>>(lv, vp);
+        else k_nms_tiles<true, 1><<<tiles, 32, 0, s>>>(lv, vp);
+    }
+    mark(ev, kStDerivNms + 1, s);
     k_hyst_unions<<<tiles, 64, 0, s>>>(lv);
     mark(ev, kStHystMerge + 1, s);
-    k_hyst_roots<<<tiles, kTileComps, 0, s>>>(lv);
+    k_hyst_roots<<<(tiles * (kTileComps / 4) + 255) / 256, 256, 0, s>>>(lv, tiles);
     k_hyst_final<<<hb, 32 * kHystWarps, 0, s>>>(lv, tiles);
     mark(ev, kStHystCompress + 1, s);
     const int tt = total_of(lv, &LevelView::thin_tiles);
@@ -1406,7 +1709,6 @@ static void launch_edges(const Levels& lv, const VoteParamsDev& vp, cudaStream_t
 void launch_image_stage(const Levels& lv, const VoteParamsDev& vp, cudaStream_t s, bool fused_pyramid,
                         cudaEvent_t* ev)
 {
-    CCTAGB_CUDA(cudaMemsetAsync(lv.cnt, 0, sizeof(LevelCounters) * lv.n, s));
     mark(ev, 0, s);
     launch_pyramid(lv, s, fused_pyramid);
     mark(ev, kStPyramid + 1, s);
@@ -1439,16 +1741,26 @@ void launch_canny_only(const Levels& lv, const VoteParamsDev& vp, cudaStream_t s
     CCTAGB_CUDA(cudaGetLastError());
 }
 
-// Edge stage of one level from its gray image (derivatives, NMS, hysteresis,
-// thinning, edge bitmap) without the compaction.  The caller clears
-// lv.cnt[0] and lv.l[0].row_count beforehand.
-__global__ void k_bitmap_to_bytes(Levels lv, uint8_t* out)
+// Edge bytes of a level's bitmap, four pixels per thread (a word each where the
+// rows are word-aligned), and the level's error bits.
+__global__ void k_bitmap_to_bytes(Levels lv, uint8_t* out, int32_t* status)
 {
     const LevelView& L = lv.l[0];
-    const size_t n = size_t(L.W) * L.H;
-    for (size_t p = size_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n; p += size_t(gridDim.x) * blockDim.x) {
-        const int x = int(p % L.W), y = int(p / L.W);
-        out[p] = edge_bit(L, x, y) ? 255 : 0;
+    const int quads = (L.W + 3) / 4;
+    const bool wide = L.W % 4 == 0 && (reinterpret_cast<size_t>(out) & 3) == 0;
+    if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = lv.cnt->err;
+    const size_t n = size_t(quads) * L.H;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
+        const int y = int(i / quads), x = 4 * int(i - size_t(y) * quads);
+        const uint32_t b = L.bitmap[size_t(y) * L.WW + (x >> 5)] >> (x & 31);
+        // bit k to byte k
+        const uint32_t v = ((b & 1u) | (b & 2u) << 7 | (b & 4u) << 14 | (b & 8u) << 21) * 0xffu;
+        uint8_t* o = out + size_t(y) * L.W + x;
+        if (wide) {
+            *reinterpret_cast<uint32_t*>(o) = v;
+        } else {
+            for (int k = 0; k < 4 && x + k < L.W; ++k) o[k] = uint8_t(v >> (8 * k));
+        }
     }
 }
 
@@ -1464,24 +1776,21 @@ void launch_scatter_counters(const LevelCounters* src, const CounterTargets& t, 
     CCTAGB_CUDA(cudaGetLastError());
 }
 
-__global__ void k_copy_status(const LevelCounters* cnt, int32_t* status)
-{
-    *status = cnt->err;
-}
-
+// Edge stage of one level from its gray image (derivatives, NMS, hysteresis,
+// thinning, edge bitmap) without the compaction; lv.l[0].row_count is null.
 void launch_edge_level(const Levels& lv, const VoteParamsDev& vp, cudaStream_t s, uint8_t* edges_out,
                        int32_t* status_out)
 {
     const LevelView& L = lv.l[0];
-    k_deriv_nms<<<L.nms_tiles, 128, 0, s>>>(lv, vp, 1);
+    k_derivs<<<L.dv_tiles, 32 * kDvWarps, 0, s>>>(lv);
     const int hb = (L.uf_tiles + kHystWarps - 1) / kHystWarps;
-    k_hyst_tiles<<<hb, 32 * kHystWarps, 0, s>>>(lv, L.uf_tiles);
+    k_nms_tiles<false, 4><<<L.uf_tiles, 128, 0, s>>>(lv, vp);  // at most 1,281 tiles
     k_hyst_unions<<<L.uf_tiles, 64, 0, s>>>(lv);
-    k_hyst_roots<<<L.uf_tiles, kTileComps, 0, s>>>(lv);
+    k_hyst_roots<<<(L.uf_tiles * (kTileComps / 4) + 255) / 256, 256, 0, s>>>(lv, L.uf_tiles);
     k_hyst_final<<<hb, 32 * kHystWarps, 0, s>>>(lv, L.uf_tiles);
     k_final_thin<<<(L.thin_tiles + kThinWarps - 1) / kThinWarps, 32 * kThinWarps, 0, s>>>(lv, L.thin_tiles);
-    k_bitmap_to_bytes<<<148 * 4, 256, 0, s>>>(lv, edges_out);
-    if (status_out) k_copy_status<<<1, 1, 0, s>>>(lv.cnt, status_out);
+    const size_t quads = size_t((L.W + 3) / 4) * L.H;
+    k_bitmap_to_bytes<<<int(std::min<size_t>((quads + 255) / 256, 148 * 8)), 256, 0, s>>>(lv, edges_out, status_out);
     CCTAGB_CUDA(cudaGetLastError());
 }
 

@@ -7,15 +7,15 @@
 // has no handle and only owns the frame and output buffers.  This entry point
 // runs the edge stage of one frame (9x9 derivatives, Canny NMS, hysteresis,
 // thinning) with the caller's input and output buffers and keeps its own
-// scratch (class map, hysteresis bit planes and tile components, edge bitmap,
-// row counts, counters) in the file-scope device array below.  It calls no
+// scratch (hysteresis bit planes and tile components, edge bitmap, counters) in
+// the file-scope device array below.  It calls no
 // cudaMalloc, cudaFree or allocating library routine.
 //
 // Limits and rules:
 //  * at most kNoAllocMaxPixels pixels and kNoAllocMaxSide per side, frame rows
 //    contiguous (pitch == width); larger frames are rejected with
 //    CCTAGB_TOO_LARGE;
-//  * the array (about 2.5 MB) is held by every GPU that loads the library,
+//  * the array (about 1.4 MB) is held by every GPU that loads the library,
 //    until the process exits;
 //  * the first call on a device (in each CUDA context: after a
 //    cudaDeviceReset the next call does it again) resolves the array's device
@@ -44,13 +44,11 @@ constexpr size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign;
 
 // Layout of the scratch array.
 constexpr size_t kOffCounters = 0;
-constexpr size_t kOffRowCount = align_up(kOffCounters + sizeof(LevelCounters));
 // bitmap words of one plane: ceil(w / 32) * h <= w h / 32 + h
 constexpr size_t kBitmapWords = size_t(kNoAllocMaxPixels) / 32 + kNoAllocMaxSide;
 // 32x32 tiles: ceil(w / 32) ceil(h / 32) <= w h / 1024 + (w + h) / 32 + 1
 constexpr size_t kMaxTiles = size_t(kNoAllocMaxPixels) / 1024 + 2 * kNoAllocMaxSide / 32 + 1;
-constexpr size_t kOffMap = align_up(kOffRowCount + sizeof(int32_t) * kNoAllocMaxSide);
-constexpr size_t kOffHyst = align_up(kOffMap + size_t(kNoAllocMaxPixels));           // 3 bitmap planes
+constexpr size_t kOffHyst = align_up(kOffCounters + sizeof(LevelCounters));             // 3 bitmap planes
 constexpr size_t kOffBlab = align_up(kOffHyst + 3 * sizeof(uint32_t) * kBitmapWords);  // 128 B per tile
 constexpr size_t kOffTcomp = align_up(kOffBlab + 128 * kMaxTiles);                     // 64 ints per tile
 constexpr size_t kOffTflag = align_up(kOffTcomp + 64 * sizeof(int32_t) * kMaxTiles);  // 64 ints per tile
@@ -135,13 +133,6 @@ extern "C" cctagb_status cctagb_edges_noalloc(const uint8_t* d_gray, int w, int 
     uint8_t* base = scratch_for_current_device(st);
     if (!base) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // What must start at zero: the counters (error bits) and the per-row edge
-    // counts the thinning kernel accumulates into.
-    if (cudaMemsetAsync(base + kOffCounters, 0, sizeof(LevelCounters), s) != cudaSuccess ||
-        cudaMemsetAsync(base + kOffRowCount, 0, sizeof(int32_t) * size_t(h), s) != cudaSuccess) {
-        cudaGetLastError();
-        return CCTAGB_CUDA_ERROR;
-    }
     Levels lv{};
     lv.n = 1;
     lv.frames = 1;
@@ -153,18 +144,15 @@ extern "C" cctagb_status cctagb_edges_noalloc(const uint8_t* d_gray, int w, int 
     L.src = const_cast<uint8_t*>(d_gray);
     L.dx = d_dx;
     L.dy = d_dy;
-    L.map = base + kOffMap;
     L.hbits = reinterpret_cast<uint32_t*>(base + kOffHyst);
     L.blab = base + kOffBlab;
     L.tcomp = reinterpret_cast<int32_t*>(base + kOffTcomp);
     L.tflag = reinterpret_cast<int32_t*>(base + kOffTflag);
     L.bitmap = reinterpret_cast<uint32_t*>(base + kOffBitmap);
-    L.row_count = reinterpret_cast<int32_t*>(base + kOffRowCount);
-    L.nms_tx = (w + 29) / 30;
-    L.nms_tiles = L.nms_tx * ((h + 29) / 30);
+    L.dv_tx = (w + 63) / 64;
+    L.dv_tiles = L.dv_tx * ((h + 63) / 64);
     L.thin_tx = (w + 31) / 32;
     L.thin_tiles = L.thin_tx * ((h + 27) / 28);  // word columns x 28-row strips
-    L.pix_blocks = int((size_t(w) * h + 255) / 256);
     L.uf_tx = (w + 31) / 32;
     L.uf_tiles = L.uf_tx * ((h + 31) / 32);
     VoteParamsDev vp{};

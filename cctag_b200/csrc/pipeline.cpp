@@ -109,7 +109,6 @@ void Pipeline::alloc(int max_w, int max_h)
         v.src = dev_alloc<uint8_t>(allocs_, px + 16);
         v.dx = dev_alloc<int16_t>(allocs_, px);
         v.dy = dev_alloc<int16_t>(allocs_, px);
-        v.map = dev_alloc<uint8_t>(allocs_, px);
         const size_t tiles = size_t((w + 31) / 32) * size_t((h + 31) / 32);
         v.hbits = dev_alloc<uint32_t>(allocs_, 3 * size_t((w + 31) / 32) * h);
         v.blab = dev_alloc<uint8_t>(allocs_, tiles * 128);
@@ -186,11 +185,10 @@ void Pipeline::set_views(int w, int h, int nl)
         v.W = w;
         v.H = h;
         v.WW = (w + 31) / 32;
-        v.nms_tx = (w + 29) / 30;
-        v.nms_tiles = v.nms_tx * ((h + 29) / 30);
+        v.dv_tx = (w + 63) / 64;
+        v.dv_tiles = v.dv_tx * ((h + 63) / 64);
         v.thin_tx = (w + 31) / 32;
         v.thin_tiles = v.thin_tx * ((h + 27) / 28);  // word columns x 28-row strips
-        v.pix_blocks = int((size_t(w) * h + 255) / 256);
         v.uf_tx = (w + 31) / 32;
         v.uf_tiles = v.uf_tx * ((h + 31) / 32);
         lv_.l[l] = v;

@@ -297,7 +297,7 @@ cctagb_status cctagb_canny_from_derivatives(cctagb_handle* h, const int16_t* dx,
  * (w*hgt bytes, 0/255) are device buffers owned by the caller; d_status (one
  * int, may be null) receives 0 or an internal error bit.  Runs asynchronously
  * on `stream` (a cudaStream_t; null = legacy default stream).  Its scratch is a
- * fixed device array inside the library (about 2.5 MB on every GPU that loads
+ * fixed device array inside the library (about 1.4 MB on every GPU that loads
  * it): frames are limited to 1,048,576 pixels and 4096 per side
  * (CCTAGB_TOO_LARGE beyond).  The first call on a device (in each CUDA
  * context) sets the array up (resolves its device address) with that device
