@@ -52,8 +52,6 @@ Detector::~Detector()
     if (h_cutpts_) cudaFreeHost(h_cutpts_);
     if (d_st1_) cudaFree(d_st1_);
     if (h_st1_) cudaFreeHost(h_st1_);
-    if (d_sel_) cudaFree(d_sel_);
-    if (d_nsel_) cudaFree(d_nsel_);
     if (ev_id0_) cudaEventDestroy(ev_id0_);
     if (ev_id1_) cudaEventDestroy(ev_id1_);
 }
@@ -162,22 +160,16 @@ void Detector::ensure_cut_capacity(int nm, int npts)
         if (h_cutin_) cudaFreeHost(h_cutin_);
         if (d_st1_) cudaFree(d_st1_);
         if (h_st1_) cudaFreeHost(h_st1_);
-        if (d_sel_) cudaFree(d_sel_);
-        if (d_nsel_) cudaFree(d_nsel_);
         d_cutin_ = nullptr;
         h_cutin_ = nullptr;
         d_st1_ = nullptr;
         h_st1_ = nullptr;
-        d_sel_ = nullptr;
-        d_nsel_ = nullptr;
         cut_cap_ = 0;
         const int cap = std::max(nm, 256);
         CCTAGB_CUDA(cudaMalloc(&d_cutin_, sizeof(CutSelectIn) * cap));
         CCTAGB_CUDA(cudaMallocHost(&h_cutin_, sizeof(CutSelectIn) * cap));
         CCTAGB_CUDA(cudaMalloc(&d_st1_, sizeof(int) * cap));
         CCTAGB_CUDA(cudaMallocHost(&h_st1_, sizeof(int) * cap));
-        CCTAGB_CUDA(cudaMalloc(&d_sel_, sizeof(int16_t) * kMaxOuterPoints * size_t(cap)));
-        CCTAGB_CUDA(cudaMalloc(&d_nsel_, sizeof(int) * cap));
         cut_cap_ = cap;
     }
     if (npts > pts_cap_) {
@@ -206,8 +198,7 @@ void Detector::select_and_identify(int nm, int npts, int w, int h)
     cp.nRefine = params_.numSamplesOuterEdgePointsRefinement;
     cp.maxSelect = std::min(params_.numCutsInIdentStep, kMaxCuts);
     cp.nOuter = params_.nSamplesOuterEllipse;
-    launch_outer_select(d_cutin_, d_cutpts_, cp.nOuter, d_sel_, d_nsel_, nm, s);
-    launch_cut_select(pipe_.level0_src(), w, h, d_cutin_, d_cutpts_, d_sel_, d_nsel_, d_tasks_, d_st1_, nm, cp, s);
+    launch_cut_select(pipe_.level0_src(), w, h, d_cutin_, d_cutpts_, d_tasks_, d_st1_, nm, cp, s);
     CCTAGB_CUDA(cudaEventRecord(ev_id0_, s));
     int maxBox = 0;
     for (int i = 0; i < nm; ++i)
@@ -220,7 +211,7 @@ void Detector::select_and_identify(int nm, int npts, int w, int h)
     CCTAGB_CUDA(cudaMemcpyAsync(h_tasks_, d_tasks_, sizeof(IdentTask) * nm, cudaMemcpyDeviceToHost, s));
     pipe_.host_wait(s);
     pipe_.add_io((long long)(sizeof(CutSelectIn) + sizeof(IdentTask)) * nm + (long long)sizeof(DirPoint) * npts,
-                 (long long)(sizeof(IdentResult) + sizeof(int) + sizeof(IdentTask)) * nm, 3);
+                 (long long)(sizeof(IdentResult) + sizeof(int) + sizeof(IdentTask)) * nm, 2);
 }
 
 namespace {

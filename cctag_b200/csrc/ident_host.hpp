@@ -66,13 +66,7 @@ std::vector<DirPoint> sorted_outer_points(const geo::Ellipse& e, const std::vect
 // status[i] (CCTAGB_ID_RELIABLE, _TOO_FEW_OUTER_POINTS, _NO_COLLECTED_CUTS or
 // _NO_SELECTED_CUTS).
 void launch_cut_select(const uint8_t* d_img, int W, int H, const CutSelectIn* d_ins, const DirPoint* d_pts,
-                       const int16_t* d_sel, const int* d_nsel, IdentTask* d_tasks, int* d_status, int n,
-                       const CutSelectParams& cp, cudaStream_t s);
-// The outer points of each marker sorted by angle and subsampled to at most
-// nOuterReq (k_outer_select): sel[i * kMaxOuterPoints + k] is the k-th
-// selected point of marker i (relative to its first), nsel[i] their number.
-void launch_outer_select(const CutSelectIn* d_ins, const DirPoint* d_pts, int nOuterReq, int16_t* d_sel, int* d_nsel,
-                         int n, cudaStream_t s);
+                       IdentTask* d_tasks, int* d_status, int n, const CutSelectParams& cp, cudaStream_t s);
 
 // Signal start along the cut as a fraction of the unit radius.
 float begin_signal(int nCrowns);
