@@ -278,7 +278,10 @@ void Detector::cut_cost(const uint8_t* d_img, int w, int h, size_t pitch, const 
     cudaStream_t s = pipe_.stream();
     CCTAGB_CUDA(cudaMemcpyAsync(d_tasks_, h_tasks_, sizeof(IdentTask) * n, cudaMemcpyHostToDevice, s));
     CCTAGB_CUDA(cudaMemcpyAsync(d_centers_, h_cost_, sizeof(float) * 2 * size_t(n), cudaMemcpyHostToDevice, s));
-    launch_cut_cost(d_img, pitch, d_tasks_, d_centers_, d_cost_, n, ident_params(params_.refineMode), s, fp64);
+    int maxCuts = 0;
+    for (int i = 0; i < n; ++i) maxCuts = std::max(maxCuts, tasks[i].ncuts);
+    launch_cut_cost(d_img, pitch, d_tasks_, d_centers_, d_cost_, n, maxCuts, ident_params(params_.refineMode), s,
+                    fp64);
     CCTAGB_CUDA(cudaMemcpyAsync(h_cost_, d_cost_, sizeof(float) * 12 * size_t(n), cudaMemcpyDeviceToHost, s));
     pipe_.host_wait(s);
     for (int i = 0; i < n; ++i) {

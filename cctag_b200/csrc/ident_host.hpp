@@ -83,9 +83,9 @@ void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_task
 // The bytes that the pixels of a marker with this outer ellipse take.
 int ident_box(float a, float b, float angle);
 // Cost and adjoints at given centers (cctagb_cut_cost): out is 12 floats per
-// task (cost, d/dcenter x2, d/dH x9).
+// task (cost, d/dcenter x2, d/dH x9); maxCuts: no task has more cuts.
 // fp64: every step in double precision (the check form of the adjoint).
 void launch_cut_cost(const uint8_t* d_img, size_t pitch, const IdentTask* d_tasks, const float* d_centers,
-                     float* d_out, int n, const IdentParams& ip, cudaStream_t s, bool fp64 = false);
+                     float* d_out, int n, int maxCuts, const IdentParams& ip, cudaStream_t s, bool fp64 = false);
 
 }  // namespace cctagb
