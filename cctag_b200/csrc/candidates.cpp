@@ -994,6 +994,8 @@ void detect_from_edges(std::vector<LevelJob>& jobs, const cctagb_params& p, cons
     }
     tasks.clear();
     for (int l = 0; l < nl; ++l) {
+        // room first: growing would copy the candidates (their move may throw)
+        st[l].loop2.reserve(size_t(std::count_if(st[l].keep.begin(), st[l].keep.end(), [](uint8_t k) { return k; })));
         for (size_t i = 0; i < st[l].keep.size(); ++i)
             if (st[l].keep[i]) st[l].loop2.push_back(std::move(st[l].loop1[i]));
         st[l].out3.assign(st[l].loop2.size(), {});

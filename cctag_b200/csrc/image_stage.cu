@@ -1469,7 +1469,7 @@ __global__ void __launch_bounds__(32 * kListWarps) k_vlists(Levels lv, VoteParam
                             L.vlist[off + k] = v[k];
                             fl = flow_step(fl, k, t[k], __frcp_rn(float(k + 1)));
                         }
-                        if (k == vp.minVotes - 1) key = v[k];
+                        if (k == max(vp.minVotes - 1, 0)) key = v[k];
                     }
                     seed = n >= vp.minVotes;
                 }

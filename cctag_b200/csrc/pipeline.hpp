@@ -30,6 +30,8 @@ struct HostLevel {
     const int32_t* vlist = nullptr;  // V
     const float* flow = nullptr;
     std::vector<int32_t> seeds;  // processing order (Multiresolution.cpp:239-242)
+    std::vector<uint64_t> voterBits;   // workspace of that order: the voters that made a seed,
+    std::vector<int32_t> votersBefore;  // and their number before each word
 };
 
 // Orders the image stages of the detectors of one handle on the GPU: each
