@@ -1027,30 +1027,51 @@ __global__ void __launch_bounds__(128) k_emit(Levels lv, int rows_total)
 // ------------------------------------------------------ gradient walk --
 // Bresenham.cpp:18-209: from an edge point, follow the gradient (dir = -1
 // backward, +1 forward) for up to distSearch steps and return the index of the
-// first edge point met, or -1.  Walk lengths spread widely (most stop within
-// two or three steps, a few run the full distance), so a warp does not run
-// one walk per lane to the end of its longest: each lane takes the next walk
-// of the warp's chunk as soon as its current one stops.  One iteration of the
-// loop below is kWalkAhead steps of a lane's walk, with the probes the
-// reference makes after each step, all loaded before the first is tested; the
-// steps and probes of every walk are those of the reference in the same order
-// (steps past the walk's end are computed and dropped), so the results do not
-// depend on the schedule.
+// first edge point met, or -1.
+//
+// Bound by the instructions of the steps (71 % of the issue slots, 19 of 32
+// lanes at work, with one loop over all steps of a walk).  Most walks stop
+// within three steps: those are taken by a lane per point for both directions
+// at once, which share the line's error terms, with all their probes in flight.
+// The others run the full distance or stop anywhere: a lane takes the next of
+// the warp's chunk as soon as its current one stops, two steps per iteration,
+// their probes loaded before the first is tested (steps past the walk's end are
+// computed and dropped).  A position is one word, x + 65536 y, so a step is one
+// addition (the sides are at most 16384); a coordinate of a walk never turns
+// back, so the side probe, which has one coordinate of this step's and one of
+// the last step's position, is inside wherever the step is.  The steps and
+// probes of every walk are those of the reference in the same order, so the
+// results do not depend on the schedule.  Measured: 1080p frame (380 k points
+// on four levels) 54 -> 32 us, 3840x2160 clutter 174 -> 110 us.
 constexpr int kWalkWarps = 8;
 constexpr int kWalkChunk = 512;  // walks (two per point) a warp takes at once, at most
-// steps a lane takes per iteration (16-frame C2 launch: 2 steps 0.50 ms, 3 steps
-// 0.52 ms; with the steps re-derived per step, 1 step 0.71 ms, 4 steps 0.69 ms,
-// 8 steps 0.92 ms: more lookahead costs occupancy)
-constexpr int kWalkAhead = 2;
 
 __device__ __forceinline__ int sgn_i(int v) { return (v > 0) - (v < 0); }
 
+// A walk step: the position moves by the major step m, and by the minor step as
+// well when the error reaches half a pixel (the return value).
+__device__ __forceinline__ bool walk_step(float& e, float a)
+{
+    e = __fadd_rn(e, a);
+    const bool c = e >= 0.5f;
+    if (c) e = __fadd_rn(e, -1.f);
+    return c;
+}
+
+// The pixel's bit of a bitidx word, and its edge point's index.
+__device__ __forceinline__ bool walk_hit(uint2 w, int at) { return __funnelshift_r(w.x, 0u, at) & 1u; }
+__device__ __forceinline__ int walk_index(uint2 w, int at, int E)
+{
+    const int idx = int(w.y) + __popc(w.x & ((1u << (at & 31)) - 1u));
+    return idx < E ? idx : -1;  // -1 past a clamped edge count
+}
+
 __global__ void __launch_bounds__(32 * kWalkWarps) k_walk(Levels lv, VoteParamsDev vp)
 {
-    __shared__ int s_xy[kWalkWarps][kWalkChunk / 2];
-    __shared__ int s_g[kWalkWarps][kWalkChunk / 2];
-    __shared__ float s_a[kWalkWarps][kWalkChunk / 2];
-    __shared__ int s_res[kWalkWarps][kWalkChunk];
+    __shared__ float s_a[kWalkWarps][kWalkChunk / 2], s_e[kWalkWarps][kWalkChunk / 2];
+    __shared__ uint8_t s_g[kWalkWarps][kWalkChunk / 2];
+    __shared__ int s_res[kWalkWarps][kWalkChunk];        // a walk's position after three steps, then its result
+    __shared__ uint16_t s_list[kWalkWarps][kWalkChunk];  // the walks that go on from there
     const unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
@@ -1067,133 +1088,128 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_walk(Levels lv, VoteParamsD
         const LevelView& L = lv.l[l];
         const int E = lv.cnt[l].E;
         const int W = L.W, H = L.H, WW = L.WW;
+        const uint2* __restrict__ bits = L.bitidx;
         const int nch = (2 * E + chunk - 1) / chunk;
         int c = (gw - first % NW + NW) % NW;
         first += nch;
+        auto inside = [&](int at) { return unsigned(at & 0xffff) < unsigned(W) && unsigned(at >> 16) < unsigned(H); };
+        auto word = [&](int at) { return __ldg(bits + ((at >> 16) * WW + ((at & 0xffff) >> 5))); };
         for (; c < nch; c += NW) {
             const int t0 = c * chunk, t1 = min(2 * E, t0 + chunk);
             const int p0 = t0 >> 1, np = (t1 - t0) >> 1;
-            // the chunk's points, |dmin / dmaj| per point (the same for both
-            // directions) and the major and minor steps of the +1 direction,
-            // (x, y) components packed as value + 1 in 2 bits each (the -1
-            // direction's are their negatives)
-            for (int i = lane; i < np; i += 32) {
-                const int xy = L.exy[p0 + i], g = L.grad[p0 + i];
-                const int gxi = int16_t(g & 0xffff), gyi = g >> 16;
-                const float gx = float(gxi), gy = float(gyi);
-                const bool ym = fabsf(gy) > fabsf(gx);
-                const int smaj = sgn_i(ym ? gyi : gxi), smin = sgn_i(ym ? gxi : gyi);
-                s_xy[wid][i] = xy;
-                s_g[wid][i] = ((ym ? 0 : smaj) + 1) | ((ym ? smaj : 0) + 1) << 2 | ((ym ? smin : 0) + 1) << 4 |
-                              ((ym ? 0 : smin) + 1) << 6;
-                s_a[wid][i] = fabsf(__fdiv_rn(ym ? gx : gy, ym ? gy : gx));
+            int ns = 0;
+            for (int i0 = 0; i0 < np; i0 += 32) {
+                const int i = i0 + lane;
+                const bool in = i < np;
+                int res[2] = {-1, -1}, at[2] = {0, 0};
+                bool more[2] = {false, false};
+                if (in) {
+                    const int xy = L.exy[p0 + i], g = L.grad[p0 + i];
+                    const int gxi = int16_t(g & 0xffff), gyi = g >> 16;
+                    const float gx = float(gxi), gy = float(gyi);
+                    const bool ym = fabsf(gy) > fabsf(gx);
+                    const int smaj = sgn_i(ym ? gyi : gxi), smin = sgn_i(ym ? gxi : gyi);
+                    // |dmin / dmaj|, the same for both directions, as is the error
+                    const float a = fabsf(__fdiv_rn(ym ? gx : gy, ym ? gy : gx));
+                    // After the first step the reference re-orients the walk
+                    // along the gradient at its start point (Bresenham.cpp:
+                    // 74-81): the direction already is dir * g, its product
+                    // with g is dir * |g|^2, so the direction stays dir * g
+                    // (0 when g is 0) and the steps are unchanged.  No probe
+                    // after the first step, and no side probe after the second.
+                    const int m = ym ? smaj * 65536 : smaj, n = ym ? smin : smin * 65536;
+                    float e = 0.f;
+                    const int d1 = m + (walk_step(e, a) ? n : 0);
+                    const int d2 = d1 + m + (walk_step(e, a) ? n : 0);
+                    const int d3 = d2 + m + (walk_step(e, a) ? n : 0);
+                    s_a[wid][i] = a;
+                    s_e[wid][i] = e;
+                    s_g[wid][i] = uint8_t((ym ? 1 : 0) | (smaj + 1) << 1 | (smin + 1) << 3);
+                    uint2 w2[2], w3[2], ws[2];
+                    bool in2[2], in3[2];
+#pragma unroll
+                    for (int d = 0; d < 2; ++d) {
+                        const int dir = d ? 1 : -1;
+                        in2[d] = inside(xy + dir * d2);
+                        in3[d] = inside(xy + dir * d3);
+                        w2[d] = w3[d] = ws[d] = make_uint2(0u, 0u);
+                        if (in2[d]) w2[d] = word(xy + dir * d2);
+                        if (in3[d]) {
+                            w3[d] = word(xy + dir * d3);
+                            ws[d] = word(xy + dir * (d3 - m));
+                        }
+                    }
+#pragma unroll
+                    for (int d = 0; d < 2; ++d) {
+                        const int dir = d ? 1 : -1;
+                        if (!in2[d]) continue;
+                        if (walk_hit(w2[d], xy + dir * d2)) {
+                            res[d] = walk_index(w2[d], xy + dir * d2, E);
+                        } else if (2 <= nmax && in3[d]) {
+                            at[d] = xy + dir * d3;
+                            if (walk_hit(w3[d], at[d])) res[d] = walk_index(w3[d], at[d], E);
+                            else if (walk_hit(ws[d], at[d] - dir * m)) res[d] = walk_index(ws[d], at[d] - dir * m, E);
+                            else more[d] = true;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int d = 0; d < 2; ++d) {
+                    if (in) s_res[wid][2 * i + d] = more[d] ? at[d] : res[d];
+                    const unsigned b = __ballot_sync(kAll, more[d]);
+                    if (more[d]) s_list[wid][ns + __popc(b & below)] = uint16_t(2 * i + d);
+                    ns += __popc(b);
+                }
             }
             __syncwarp();
-            int q = t0, t = 0, x = 0, y = 0, n = 0;
-            int mx = 0, my = 0, nx = 0, ny = 0;  // major and minor step (the side probe is one major step back)
+            int q = 0, t = 0, at = 0, n = 0, m = 0, mn = 0;  // major step; major and minor step
             float e = 0.f, a = 0.f;
             bool act = false;
             while (true) {
                 const unsigned idle = __ballot_sync(kAll, !act);
                 if (!act) {
                     const int k = q + __popc(idle & below);
-                    if (k < t1) {
-                        t = k;
+                    if (k < ns) {
+                        t = s_list[wid][k];
                         act = true;
-                        const int i = (k - t0) >> 1;
-                        const int xy = s_xy[wid][i], st = s_g[wid][i];
-                        const int dir = (k & 1) ? 1 : -1;
-                        x = xy & 0xffff;
-                        y = xy >> 16;
-                        mx = dir * ((st & 3) - 1);
-                        my = dir * ((st >> 2 & 3) - 1);
-                        nx = dir * ((st >> 4 & 3) - 1);
-                        ny = dir * ((st >> 6 & 3) - 1);
+                        const int i = t >> 1, st = s_g[wid][i], dir = (t & 1) ? 1 : -1;
+                        const int maj = dir * ((st >> 1 & 3) - 1), min_ = dir * ((st >> 3) - 1);
+                        m = st & 1 ? maj * 65536 : maj;
+                        mn = m + (st & 1 ? min_ : min_ * 65536);
+                        at = s_res[wid][t];
                         a = s_a[wid][i];
-                        e = 0.f;
-                        n = 0;
+                        e = s_e[wid][i];
+                        n = 3;
                     }
                 }
                 q += __popc(idle);
                 if (!__any_sync(kAll, act)) break;
                 if (!act) continue;
-                // The next kWalkAhead steps of the walk: its positions do not
-                // depend on what the probes find, so all their probes are
-                // issued before the first is looked at.  kind: 0 a step without
-                // a probe, 1 one probe, 2 a probe and the side probe, 3 the
-                // walk ends here (distSearch), 4 past the end.
-                int kind[kWalkAhead], px[kWalkAhead], py[kWalkAhead], sx[kWalkAhead], sy[kWalkAhead];
-                bool over = false;
-#pragma unroll
-                for (int j = 0; j < kWalkAhead; ++j) {
-                    kind[j] = 4;
-                    px[j] = py[j] = sx[j] = sy[j] = -1;
-                    if (over) continue;
-                    if (n >= 2 && n > nmax) {
-                        kind[j] = 3;
-                        over = true;
-                        continue;
-                    }
-                    e = __fadd_rn(e, a);
-                    x += mx;
-                    y += my;
-                    if (e >= 0.5f) {
-                        x += nx;
-                        y += ny;
-                        e = __fadd_rn(e, -1.f);
-                    }
-                    ++n;
-                    // After the first step the reference re-orients the walk
-                    // along the gradient at its start point (Bresenham.cpp:
-                    // 74-81): the direction already is dir * g, its product
-                    // with g is dir * |g|^2, so the direction stays dir * g
-                    // (0 when g is 0) and the steps are unchanged.
-                    if (n == 1) {
-                        kind[j] = 0;
-                    } else {
-                        kind[j] = n > 2 ? 2 : 1;
-                        px[j] = x;
-                        py[j] = y;
-                        sx[j] = x - mx;
-                        sy[j] = y - my;
-                    }
+                // the walk ends before a step once n > nmax
+                const int a0 = at + (walk_step(e, a) ? mn : m), a1 = a0 + (walk_step(e, a) ? mn : m);
+                const bool in0 = inside(a0) && n <= nmax, in1 = inside(a1) && n < nmax;
+                uint2 w0 = make_uint2(0u, 0u), w1 = w0, v0 = w0, v1 = w0;
+                if (in0) {
+                    w0 = word(a0);
+                    v0 = word(a0 - m);
                 }
-                uint2 w[kWalkAhead], ws[kWalkAhead];
-#pragma unroll
-                for (int j = 0; j < kWalkAhead; ++j) {
-                    w[j] = ws[j] = make_uint2(0u, 0u);
-                    if (kind[j] == 1 || kind[j] == 2) {
-                        if (unsigned(px[j]) < unsigned(W) && unsigned(py[j]) < unsigned(H))
-                            w[j] = __ldg(&L.bitidx[size_t(py[j]) * WW + (px[j] >> 5)]);
-                        if (kind[j] == 2 && unsigned(sx[j]) < unsigned(W) && unsigned(sy[j]) < unsigned(H))
-                            ws[j] = __ldg(&L.bitidx[size_t(sy[j]) * WW + (sx[j] >> 5)]);
-                    }
+                if (in1) {
+                    w1 = word(a1);
+                    v1 = word(a1 - m);
                 }
-                // the first step, in walk order, that ends the walk: -1
-                // outside the level or at distSearch, else the index of the
-                // edge pixel met (-1 past a clamped edge count)
-                auto found = [&](uint2 v, int qx, int qy) -> int {
-                    if (unsigned(qx) >= unsigned(W) || unsigned(qy) >= unsigned(H)) return -1;
-                    const uint32_t bit = 1u << (qx & 31);
-                    if (!(v.x & bit)) return -2;
-                    const int idx = int(v.y) + __popc(v.x & (bit - 1u));
-                    return idx < E ? idx : -1;
-                };
-                int res = -2;  // -2: the walk goes on
-#pragma unroll
-                for (int j = 0; j < kWalkAhead; ++j) {
-                    if (res != -2) continue;
-                    if (kind[j] == 3) {
-                        res = -1;
-                    } else if (kind[j] == 1 || kind[j] == 2) {
-                        res = found(w[j], px[j], py[j]);
-                        if (res == -2 && kind[j] == 2) res = found(ws[j], sx[j], sy[j]);
-                    }
-                }
-                if (res != -2) {
-                    s_res[wid][t - t0] = res;
+                const bool f0 = walk_hit(w0, a0), g0 = walk_hit(v0, a0 - m);
+                const bool f1 = walk_hit(w1, a1), g1 = walk_hit(v1, a1 - m);
+                if (!in1 || f0 || g0 || f1 || g1) {
+                    int res = -1;
+                    if (f0) res = walk_index(w0, a0, E);
+                    else if (g0) res = walk_index(v0, a0 - m, E);
+                    else if (f1) res = walk_index(w1, a1, E);
+                    else if (g1) res = walk_index(v1, a1 - m, E);
+                    s_res[wid][t] = res;
                     act = false;
                 }
+                at = a1;
+                n += 2;
             }
             __syncwarp();
             for (int i = lane; i < np; i += 32) {
