@@ -1082,6 +1082,10 @@ __global__ void __maxnreg__(72)
         }
         return;
     }
+    // A block's shared memory may be reached from another one once it runs: each
+    // arrives here (the return above is taken by whole clusters) and waits before
+    // the rounds, whose shares go to every block, behind the set-up and staging.
+    if constexpr (CLUSTER) cg::this_cluster().barrier_arrive();
 
     if (tid == 0) {
         canonic_form(T.Q, S.C, S.Tp, S.Td);
@@ -1138,6 +1142,7 @@ __global__ void __maxnreg__(72)
     Tasks K{nTrials, nS / kChunk, nS % kChunk, 1, 0};
     while (K.width < K.tail) K.width <<= 1;
     K.packed = kChunk / K.width;
+    if constexpr (CLUSTER) cg::this_cluster().barrier_wait();
     float ns = ip.neighbourSize;
     for (int round = 0; round < S.rounds; ++round) {
         // getNearbyPoints (Identification.cpp:1071-1109): a lane per trial
