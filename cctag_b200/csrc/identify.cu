@@ -2081,8 +2081,9 @@ void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_task
     const int warps = cluster == kMaxCluster ? 10 : perSm == 1 ? kMaxIdWarps : perSm == 2 ? 12 : kMaxChunks;
     // Dynamic shared memory: the lines or the Gauss-Newton samples, then the
     // pixels of the largest marker, as far as they fit (1 KB per block is the
-    // driver's).
-    size_t work = grid_work(ip.gridN * ip.gridN, std::min(maxCuts, kMaxCuts));
+    // driver's; markers without cuts, as numCutsInIdentStep <= 0 leaves them,
+    // take none).
+    size_t work = grid_work(ip.gridN * ip.gridN, std::min(std::max(maxCuts, 0), kMaxCuts));
     if (gn && warps > kMaxChunks) work = std::max(work, kGnWork);
     const size_t fixed = align16(sizeof(Shared)) + work + 1024;
     const size_t room = std::min(size_t(smemBlock), size_t(smemSm) / size_t(perSm)) - fixed;
