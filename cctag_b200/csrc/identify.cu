@@ -39,6 +39,7 @@
 
 #include "common.hpp"
 #include "ident_host.hpp"
+#include "ident_layout.hpp"
 #include "cctag_b200/portable/pmath.hpp"
 
 namespace cctagb {
@@ -53,9 +54,7 @@ constexpr int kWarps = kThreads / 32;
 // all layouts give the same bits.
 constexpr int kChunk = 32;
 constexpr int kMaxChunks = kMaxSamples / kChunk;
-constexpr int kMaxCluster = 8;      // blocks per marker at most
-constexpr int kMaxIdWarps = 20;     // warps per block of k_identify at most
-constexpr int kGnBlocks = 7;        // blocks per SM of a large Gauss-Newton launch
+static_assert(kGnWarps == kMaxChunks, "a warp per chunk");
 
 __device__ __forceinline__ void mat_mul(const float* a, const float* b, float* r)
 {
@@ -216,7 +215,9 @@ struct GnChunk {  // Gauss-Newton, one chunk of samples
     float dx[kMaxCuts][kChunk];           // d value / d center x
     float dy[kMaxCuts][kChunk];           // d value / d center y
 };
-constexpr int kGnWhole = 2400;            // cuts x samples whose values and derivatives fit at once
+// Cuts x samples whose values and derivatives Gauss-Newton has room for at least;
+// a block with an SM to itself has it for all of its marker's.
+constexpr int kGnWhole = 2400;
 constexpr int kSigStride = kMaxSamples + 1;
 // What the reading of the cuts keeps once the center is found.
 struct FinalWork {
@@ -838,7 +839,7 @@ __device__ __forceinline__ void gn_chunk_sums(uint32_t valid, int n, bool live, 
 // the damping raised.  Stops when a step is below 1e-3 px, or after
 // gnIterations cost evaluations.
 template <bool CLUSTER>
-__device__ void gn_refine(Shared& S, void* work, const uint8_t* px, const IdentTask& T, const Roi& roi,
+__device__ void gn_refine(Shared& S, void* work, int room, const uint8_t* px, const IdentTask& T, const Roi& roi,
                           const IdentParams& ip, uint32_t cutMask, int crank, int csize)
 {
     namespace cg = cooperative_groups;
@@ -935,10 +936,10 @@ __device__ void gn_refine(Shared& S, void* work, const uint8_t* px, const IdentT
                     for (int q = 0; q < 6; ++q) S.gPart[par][j][q] = acc[q];
             }
             __syncthreads();
-        } else if (!CLUSTER && T.ncuts * nS <= kGnWhole) {
+        } else if (!CLUSTER && T.ncuts * nS <= room) {
             float* gs = static_cast<float*>(work);
-            float* gdx = gs + kGnWhole;
-            float* gdy = gdx + kGnWhole;
+            float* gdx = gs + room;
+            float* gdy = gdx + room;
             for (int i = tid; i < T.ncuts * nS; i += nthreads) {
                 const int c = i / nS;
                 if (!((valid >> c) & 1u)) continue;
@@ -1233,7 +1234,7 @@ __global__ void __maxnreg__(72)
         ns /= float((gridN - 1) / 2);
     }
     if (ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON && !S.fail && S.rounds > 0)
-        gn_refine<CLUSTER>(S, work, px, T, roi, ip, cutMask, crank, csize);
+        gn_refine<CLUSTER>(S, work, workBytes / int(3 * sizeof(float)), px, T, roi, ip, cutMask, crank, csize);
     const bool read = !S.fail && S.rounds > 0;
     IdentResult& R = res[marker];
     if (!read && tid == 0 && crank == 0) {
@@ -2052,19 +2053,9 @@ void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_task
         throw Error{CCTAGB_BAD_ARG, "gnIterations must be in [1, 100]"};
     if (ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON && (ip.coarseRounds < 1 || ip.coarseRounds > 64))
         throw Error{CCTAGB_BAD_ARG, "gnCoarseRounds must be in [1, 64]"};
-    // Blocks per marker and warps per block.  A round has one task per trial
-    // and chunk of 32 samples, 79 for 25 trials of 100 samples (the partial
-    // chunks packed): with few markers they spread over a cluster of 8 blocks
-    // of 10 warps, then 4 or 2 blocks of 20, as long as the markers' blocks
-    // (nearly) fit the SMs side by side: a marker's time grows with its size,
-    // so the few blocks beyond start as the smallest markers end.  With more
-    // markers a block each, of 20 warps while an SM has one marker, else two
-    // blocks of 12 warps on an SM, or for Gauss-Newton, most of whose time is
-    // serial steps of a marker, kGnBlocks of 4.  The block layout keeps to one
-    // block per marker, which takes the least SM time.
     // Measured, against a block of 25 warps per marker (a cluster of 4 below 38
     // markers) that read the image and one trial per warp: 28 markers of a 1080p
-    // frame 261 -> 120 us, 80 of a 3840x2160 clutter frame 588 -> 377 us, 1024
+    // frame 261 -> 120 us, 80 of a 3840x2160 clutter frame 588 -> 383 us, 1024
     // candidates of 8-150 px radius 3.15 -> 1.48 ms (1.95 ms in the caller's
     // order), by Gauss-Newton 4096 of them 2.61 -> 1.65 ms (4 to 6 blocks per SM,
     // with room for larger markers' pixels, 3 % slower).
@@ -2074,17 +2065,17 @@ void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_task
     CCTAGB_CUDA(cudaDeviceGetAttribute(&smemBlock, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     CCTAGB_CUDA(cudaDeviceGetAttribute(&smemSm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     const bool gn = ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON;
-    int cluster = 1;
-    if (ip.layout != CCTAGB_IDENT_BLOCK)
-        for (cluster = kMaxCluster; cluster > 1 && n * cluster > sms + (cluster == 2 ? sms / 4 : 0);) cluster >>= 1;
-    const int perSm = cluster > 1 || n <= sms ? 1 : gn && n > 2 * sms ? kGnBlocks : 2;
-    const int warps = cluster == kMaxCluster ? 10 : perSm == 1 ? kMaxIdWarps : perSm == 2 ? 12 : kMaxChunks;
+    const auto [cluster, perSm, warps] =
+        ident_layout(n, sms, (ip.nSamples + kChunk - 1) / kChunk, gn, ip.layout == CCTAGB_IDENT_BLOCK);
     // Dynamic shared memory: the lines or the Gauss-Newton samples, then the
     // pixels of the largest marker, as far as they fit (1 KB per block is the
     // driver's; markers without cuts, as numCutsInIdentStep <= 0 leaves them,
     // take none).
-    size_t work = grid_work(ip.gridN * ip.gridN, std::min(std::max(maxCuts, 0), kMaxCuts));
-    if (gn && warps > kMaxChunks) work = std::max(work, kGnWork);
+    const int cuts = std::min(std::max(maxCuts, 0), kMaxCuts);
+    size_t work = grid_work(ip.gridN * ip.gridN, cuts);
+    if (gn && warps > kMaxChunks)
+        work = std::max({work, kGnWork,
+                         cluster == 1 && perSm == 1 ? align16(3 * sizeof(float) * size_t(cuts * ip.nSamples)) : 0});
     const size_t fixed = align16(sizeof(Shared)) + work + 1024;
     const size_t room = std::min(size_t(smemBlock), size_t(smemSm) / size_t(perSm)) - fixed;
     const size_t box = std::min(align16(size_t(std::max(maxBox, 0))), room & ~size_t(15));
