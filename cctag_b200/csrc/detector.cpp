@@ -139,12 +139,9 @@ void Detector::identify_on(const uint8_t* d_img, size_t pitch, const IdentTask* 
     cudaStream_t s = pipe_.stream();
     CCTAGB_CUDA(cudaMemcpyAsync(d_tasks_, h_tasks_, sizeof(IdentTask) * n, cudaMemcpyHostToDevice, s));
     CCTAGB_CUDA(cudaEventRecord(ev_id0_, s));
-    int maxCuts = 1, maxBox = 0;
-    for (int i = 0; i < n; ++i) {
-        maxCuts = std::max(maxCuts, tasks[i].ncuts);
-        maxBox = std::max(maxBox, ident_box(tasks[i].a, tasks[i].b, tasks[i].angle));
-    }
-    launch_identify(d_img, pitch, d_tasks_, d_res_, n, maxCuts, maxBox, d_bank_inv_, ip, s);
+    int maxCuts = 1;
+    for (int i = 0; i < n; ++i) maxCuts = std::max(maxCuts, tasks[i].ncuts);
+    launch_identify(d_img, pitch, d_tasks_, d_res_, n, tasks, maxCuts, d_bank_inv_, ip, s);
     CCTAGB_CUDA(cudaEventRecord(ev_id1_, s));
     CCTAGB_CUDA(cudaMemcpyAsync(h_res_, d_res_, sizeof(IdentResult) * n, cudaMemcpyDeviceToHost, s));
     pipe_.host_wait(s);
@@ -200,10 +197,7 @@ void Detector::select_and_identify(int nm, int npts, int w, int h)
     cp.nOuter = params_.nSamplesOuterEllipse;
     launch_cut_select(pipe_.level0_src(), w, h, d_cutin_, d_cutpts_, d_tasks_, d_st1_, nm, cp, s);
     CCTAGB_CUDA(cudaEventRecord(ev_id0_, s));
-    int maxBox = 0;
-    for (int i = 0; i < nm; ++i)
-        maxBox = std::max(maxBox, ident_box(h_tasks_[i].a, h_tasks_[i].b, h_tasks_[i].angle));
-    launch_identify(pipe_.level0_src(), size_t(w), d_tasks_, d_res_, nm, cp.maxSelect, maxBox, d_bank_inv_,
+    launch_identify(pipe_.level0_src(), size_t(w), d_tasks_, d_res_, nm, h_tasks_, cp.maxSelect, d_bank_inv_,
                     ident_params(params_.refineMode), s);
     CCTAGB_CUDA(cudaEventRecord(ev_id1_, s));
     CCTAGB_CUDA(cudaMemcpyAsync(h_res_, d_res_, sizeof(IdentResult) * nm, cudaMemcpyDeviceToHost, s));

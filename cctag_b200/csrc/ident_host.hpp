@@ -74,12 +74,13 @@ float begin_signal(int nCrowns);
 // Device side (identify.cu).  The bank lives in a device buffer of
 // kMaxBankIds x kMaxBankRatios floats (1 / ratio) owned by the caller.
 void upload_bank(const std::vector<std::vector<float>>& bank, float* d_bank_inv);
-// Tasks carry their image rectangle; d_img rows are pitch bytes apart.  maxCuts
-// bounds the tasks' ncuts; maxBox is the room in bytes wanted for a marker's
-// pixels in shared memory (ident_box; a marker that needs more than there is
-// reads the image instead, with the same results).
+// Tasks carry their image rectangle; d_img rows are pitch bytes apart.  tasks: the
+// host's copy (their ellipses are read, for the room that their pixels take in
+// shared memory; a marker that needs more reads the image instead, with the same
+// results); maxCuts bounds the launched tasks' ncuts.
 void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_tasks, IdentResult* d_res, int n,
-                     int maxCuts, int maxBox, const float* d_bank_inv, const IdentParams& ip, cudaStream_t s);
+                     const IdentTask* tasks, int maxCuts, const float* d_bank_inv, const IdentParams& ip,
+                     cudaStream_t s);
 // The bytes that the pixels of a marker with this outer ellipse take.
 int ident_box(float a, float b, float angle);
 // Cost and adjoints at given centers (cctagb_cut_cost): out is 12 floats per

@@ -47,6 +47,7 @@ namespace cctagb {
 namespace {
 
 constexpr int kMaxTrials = 25;
+static_assert(kIdentTrialWarps == kMaxTrials, "a warp per trial");
 constexpr int kThreads = 32 * kMaxTrials;  // of the cost kernels
 constexpr int kWarps = kThreads / 32;
 // The samples along a cut come in chunks of 32 (one per lane).  Per-chunk sums
@@ -592,6 +593,57 @@ __device__ __forceinline__ double trial_tail(const TrialLines& lines, const Samp
     return v;
 }
 
+// The same shares of all chunks of a trial, for pixels read from the image: the
+// reads of a cut's chunks overlap, two cuts at a time.  Lanes past the last sample
+// read it again (in bounds, no branch) and contribute zero.
+__device__ __forceinline__ void trial_chunks(const TrialLines& lines, const SampleArea<false>& A, int t,
+                                             uint32_t valid, int samples, int lane, double out[kMaxChunks])
+{
+    constexpr int G = 2;  // cuts per step
+    const int n = __popc(valid);
+    float v0[kMaxChunks], s1[kMaxChunks], s2[kMaxChunks], kf[kMaxChunks];
+#pragma unroll
+    for (int q = 0; q < kMaxChunks; ++q) {
+        kf[q] = float(min(q * kChunk + lane, samples - 1));
+        v0[q] = s1[q] = s2[q] = 0.f;
+    }
+    if (n >= 2) {
+        bool first = true;
+        for (uint32_t m = valid; m;) {
+            const int have = __popc(m);
+            float val[G][kMaxChunks];
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int i = t * lines.stride + (m ? __ffs(m) - 1 : 0);  // past the last valid cut: read, not used
+                m &= m - 1;
+                const float4 l = lines.uv[i];
+                const float2 lw = lines.w[i];
+#pragma unroll
+                for (int q = 0; q < kMaxChunks; ++q) val[g][q] = cut_sample(A, l, lw, kf[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < kMaxChunks; ++q)
+                if (first) v0[q] = val[0][q];  // first valid cut: the shift
+            first = false;
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                if (g >= have) break;
+#pragma unroll
+                for (int q = 0; q < kMaxChunks; ++q) {
+                    const float d = __fsub_rn(val[g][q], v0[q]);
+                    s1[q] = __fadd_rn(s1[q], d);
+                    s2[q] = __fmaf_rn(d, d, s2[q]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kMaxChunks; ++q)
+        out[q] = lane_sum(n >= 2 && q * kChunk + lane < samples
+                              ? kTermScale * double(__fsub_rn(__fmul_rn(float(n), s2[q]), __fmul_rn(s1[q], s1[q])))
+                              : 0.0);
+}
+
 // The sampling tasks of a round, spread over the warps of the cluster: one per
 // trial and whole chunk, chunk by chunk (a block keeps to a band of the
 // marker), then the packed partial chunks; `valid` is trial `lane`'s cuts.
@@ -1045,9 +1097,10 @@ __device__ void gn_refine(Shared& S, void* work, int room, const uint8_t* px, co
 }  // namespace
 
 // One marker per cluster (CLUSTER, blocks of one marker side by side) or per
-// block; any number of warps.  72 registers: 25 warps on an SM put 7 on one of
-// its four register partitions (five blocks of 5 warps, or one of 20).
-template <bool CLUSTER>
+// block; any number of warps up to kIdentTrialWarps.  72 registers: 25 warps on an SM put 7
+// on one of its four register partitions (one block of 25, or two of 12).
+// TRIALS: one block per marker with a warp per trial, no pixels staged (grid only).
+template <bool CLUSTER, bool TRIALS>
 __global__ void __maxnreg__(72)
     k_identify(const uint8_t* __restrict__ img, size_t pitch, const IdentTask* __restrict__ tasks, IdentResult* res,
                const float* __restrict__ bankInv, IdentParams ip, int workBytes, int boxBytes)
@@ -1188,8 +1241,17 @@ __global__ void __maxnreg__(72)
         const uint32_t valid = lane < nTrials ? ~flags & cutMask : 0u;
         const int par = round & 1;
         const int firstTask = crank * nwarps + warp, stepTask = csize * nwarps;
-        if (S.direct) sample_round(S, lines, image_area(roi), K, valid, par, firstTask, stepTask, csize, lane);
-        else sample_round(S, lines, staged_area(S, px), K, valid, par, firstTask, stepTask, csize, lane);
+        if constexpr (TRIALS) {
+            double c[kMaxChunks];
+            trial_chunks(lines, image_area(roi), warp, __shfl_sync(0xffffffffu, valid, warp), nS, lane, c);
+#pragma unroll
+            for (int q = 0; q < kMaxChunks; ++q)
+                if (lane == 0) S.part[par][q][warp] = c[q];
+        } else if (S.direct) {
+            sample_round(S, lines, image_area(roi), K, valid, par, firstTask, stepTask, csize, lane);
+        } else {
+            sample_round(S, lines, staged_area(S, px), K, valid, par, firstTask, stepTask, csize, lane);
+        }
         // All chunks of the marker are in, in every block; this parity's array
         // is written again two rounds later, after the next cluster barrier,
         // when every block has finished reading it.
@@ -1233,7 +1295,7 @@ __global__ void __maxnreg__(72)
         if (S.fail) break;
         ns /= float((gridN - 1) / 2);
     }
-    if (ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON && !S.fail && S.rounds > 0)
+    if (!TRIALS && ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON && !S.fail && S.rounds > 0)
         gn_refine<CLUSTER>(S, work, workBytes / int(3 * sizeof(float)), px, T, roi, ip, cutMask, crank, csize);
     const bool read = !S.fail && S.rounds > 0;
     IdentResult& R = res[marker];
@@ -2041,7 +2103,7 @@ void upload_bank(const std::vector<std::vector<float>>& bank, float* d_bank_inv)
 }
 
 void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_tasks, IdentResult* d_res, int n,
-                     int maxCuts, int maxBox, const float* d_bank_inv, const IdentParams& ip, cudaStream_t s)
+                     const IdentTask* tasks, int maxCuts, const float* d_bank_inv, const IdentParams& ip, cudaStream_t s)
 {
     if (n <= 0) return;
     if (ip.gridN * ip.gridN > kMaxTrials || ip.gridN < 3 || (ip.gridN & 1) == 0)
@@ -2065,22 +2127,55 @@ void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_task
     CCTAGB_CUDA(cudaDeviceGetAttribute(&smemBlock, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     CCTAGB_CUDA(cudaDeviceGetAttribute(&smemSm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     const bool gn = ip.refineMode == CCTAGB_REFINE_GAUSS_NEWTON;
-    const auto [cluster, perSm, warps] =
-        ident_layout(n, sms, (ip.nSamples + kChunk - 1) / kChunk, gn, ip.layout == CCTAGB_IDENT_BLOCK);
     // Dynamic shared memory: the lines or the Gauss-Newton samples, then the
-    // pixels of the largest marker, as far as they fit (1 KB per block is the
-    // driver's; markers without cuts, as numCutsInIdentStep <= 0 leaves them,
-    // take none).
+    // markers' pixels (1 KB per block is the driver's; markers without cuts, as
+    // numCutsInIdentStep <= 0 leaves them, take none).
     const int cuts = std::min(std::max(maxCuts, 0), kMaxCuts);
     size_t work = grid_work(ip.gridN * ip.gridN, cuts);
-    if (gn && warps > kMaxChunks)
-        work = std::max({work, kGnWork,
-                         cluster == 1 && perSm == 1 ? align16(3 * sizeof(float) * size_t(cuts * ip.nSamples)) : 0});
-    const size_t fixed = align16(sizeof(Shared)) + work + 1024;
-    const size_t room = std::min(size_t(smemBlock), size_t(smemSm) / size_t(perSm)) - fixed;
-    const size_t box = std::min(align16(size_t(std::max(maxBox, 0))), room & ~size_t(15));
+    auto room = [&](int perSm) {
+        const size_t all = std::min(size_t(smemBlock), size_t(smemSm) / size_t(perSm));
+        return (all - align16(sizeof(Shared)) - work - 1024) & ~size_t(15);
+    };
+    struct {
+        size_t largest = 0, some = 0;  // largest marker's pixels, of those that leave kIdentSpareL1
+        int beyond = 0, half = 0;      // markers whose pixels exceed `one`, `two` bytes
+    } px;
+    auto look = [&](size_t one, size_t two) {
+        for (int i = 0; i < n; ++i) {
+            const size_t b = align16(size_t(ident_box(tasks[i].a, tasks[i].b, tasks[i].angle)));
+            px.largest = std::max(px.largest, b);
+            if (b + kIdentSpareL1 <= one) px.some = std::max(px.some, b);
+            px.beyond += b > one ? 1 : 0;
+            px.half += b > two ? 1 : 0;
+        }
+    };
+    IdentLaunch a{n, sms, ip.gridN * ip.gridN, ip.nSamples, gn, ip.layout == CCTAGB_IDENT_BLOCK, 0, 0};
+    if (!gn) {
+        look(room(1), room(2));
+        a.beyond = px.beyond;
+        a.beyondHalf = px.half;
+    }
+    IdentLayout l = ident_layout(a);
+    const int cluster = l.cluster, perSm = l.perSm, warps = l.warps;
+    if (gn) {
+        if (warps > kMaxChunks)
+            work = std::max({work, kGnWork,
+                             cluster == 1 && perSm == 1 ? align16(3 * sizeof(float) * size_t(cuts * ip.nSamples)) : 0});
+        look(room(perSm), room(perSm));
+        // reads take less of a marker's time than in the grid: room is kept while a
+        // third of the markers use it (4096 of 8-200 px, 68 % beyond: 2.00 ms with,
+        // 1.94 without; 400 of 8-150 px, 52 % beyond: 322 and 333 us), but a launch
+        // of one wave lasts as long as its largest marker (92 of 200 and 400 px 217
+        // and 193 us)
+        if (3LL * px.beyond > 2LL * n || (px.beyond && cluster == 1 && n <= sms)) l.pixels = IdentPixels::kNone;
+    }
+    const size_t box = l.pixels == IdentPixels::kNone   ? 0
+                       : l.pixels == IdentPixels::kSome ? px.some
+                                                        : std::min(px.largest, room(perSm));
     const size_t smem = std::max(work + box, sizeof(FinalWork));
-    auto* kernel = cluster > 1 ? k_identify<true> : k_identify<false>;
+    auto* kernel = cluster > 1                 ? k_identify<true, false>
+                   : warps == kIdentTrialWarps ? k_identify<false, true>
+                                               : k_identify<false, false>;
     CCTAGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      smemBlock - int(align16(sizeof(Shared)))));
     cudaLaunchConfig_t cfg = {};
