@@ -1554,9 +1554,10 @@ struct CostShared {
 };
 
 // A sample's image point under H, and 1 / w.  The two quotients by one rounded
-// reciprocal and a remainder step each (pm::div_small's, correctly rounded: a
-// finite, nonzero determinant, as the caller has, keeps them far from the ends
-// of the range).
+// reciprocal and a remainder step each (pm::div_small's, for any divisor).  An
+// invertible H has a line that it sends to infinity: a sample on it, or so near that
+// 1 / w overflows, gets NaN or an infinity, which inside() refuses, so its cut is
+// dropped, as with the quotient itself (an infinity, or beyond any image).
 __device__ __forceinline__ void cost_point(const float* H, float x, float y, float& qx, float& qy, float& rw)
 {
     const float u = H[0] * x + H[1] * y + H[2];

@@ -118,6 +118,11 @@ CCTAGB_HD inline double atan2_d(double y, double x)
 // "Computation of elementary functions on the IBM RISC System/6000
 // processor", IBM J. Res. Dev. 34(1), 1990).  Valid while x, q and r stay
 // normal; checked exhaustively over a binade of x for every d in [1, 256].
+// For other divisors q may be half an ulp further off where |x|'s significand is
+// the smaller one, past the theorem's premise; no quotient differed from x / d in
+// tests/cpp/div_general_test.cpp (random pairs, and a binade of x for divisors
+// next to the powers of two).  A zero d, or one whose reciprocal overflows, gives
+// NaN or an infinity.
 // Three dependent operations instead of a full division.
 CCTAGB_HD inline float div_small(float x, float d, float y)
 {
