@@ -51,7 +51,7 @@ struct IdentLaunch {
 // pairs up to a quarter beyond: the pairs that start late cost where all markers
 // are alike (92 of 50 px radius 327 us, a block each 253; 75 of 8-150 px 292 and
 // 297), but a block each leaves a large one to a single SM (80 candidates of a
-// 3840x2160 clutter frame, of up to 300 px, 387 us in pairs, 664 a block each).
+// 3840x2160 clutter frame, of up to 300 px, 346 us in pairs, 547 a block each).
 // With more markers a block each, of 20 warps while an SM has one marker, else two
 // blocks of 12 warps on an SM.
 //

@@ -2118,7 +2118,7 @@ void launch_identify(const uint8_t* d_img, size_t pitch, const IdentTask* d_task
         throw Error{CCTAGB_BAD_ARG, "gnCoarseRounds must be in [1, 64]"};
     // Measured, against a block of 25 warps per marker (a cluster of 4 below 38
     // markers) that read the image and one trial per warp: 28 markers of a 1080p
-    // frame 261 -> 120 us, 80 of a 3840x2160 clutter frame 588 -> 383 us, 1024
+    // frame 261 -> 120 us, 80 of a 3840x2160 clutter frame 588 -> 346 us, 1024
     // candidates of 8-150 px radius 3.15 -> 1.48 ms (1.95 ms in the caller's
     // order), by Gauss-Newton 4096 of them 2.61 -> 1.65 ms (4 to 6 blocks per SM,
     // with room for larger markers' pixels, 3 % slower).
