@@ -1149,7 +1149,9 @@ __global__ void __maxnreg__(72)
         float mT[9] = {sqrt2 / meanAB, 0.f, -sqrt2 * T.cx / meanAB, 0.f, sqrt2 / meanAB, -sqrt2 * T.cy / meanAB,
                        0.f, 0.f, 1.f};
         float mTi[9];
-        mat_inv(mT, mTi);
+        // no conditioner for axes of no or unlimited mean: no trial center then
+        if (!mat_inv(mT, mTi))
+            for (int k = 0; k < 9; ++k) mTi[k] = NAN;
         float tq[9], Qc[9], mTiT[9];
         for (int i = 0; i < 3; ++i)
             for (int j = 0; j < 3; ++j) mTiT[i * 3 + j] = mTi[j * 3 + i];
